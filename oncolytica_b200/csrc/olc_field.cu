@@ -545,6 +545,7 @@ bool make_field_maps(FieldMaps* m, float* a, float* b, const int dims[3], int ti
     m->keep = (int)((long long)dims[2] * keep_pct / 100);
     m->VY = tile_y;
     m->VZ = tile_z;
+    m->passes = tile_y != 8 || tile_z != 8 || pair_threads > 0 || keep_pct > 0;
     const cuuint32_t boxv[3] = {72, (cuuint32_t)(tile_y + 2), (cuuint32_t)(tile_z + 2)};
     if (!encode_map(&m->vec[0], a, dims, boxv) || !encode_map(&m->vec[1], b, dims, boxv)) return false;
     m->ok = true;
@@ -679,6 +680,13 @@ float* run_substeps_tma(float* a, float* b, const FieldMaps& m, int a_index, con
     bufs[1 - a_index] = b;
     int cur = a_index;
     int i = 0;
+    if (!m.passes && !(pins && pins->n) && resident_fits(fs)) {
+        for (; i < RESIDENT_LEAD; ++i) {
+            launch_single(m, cur, bufs[1 - cur], fs, status, i & 1, s);
+            cur = 1 - cur;
+        }
+        if (float* res = run_resident(bufs[cur], bufs[1 - cur], fs, fs.substeps - i, status, s)) return res;
+    }
     if (m.pair_nt && !(pins && pins->n)) {
         // two substeps per launch (pinned voxels are re-pinned after every
         // substep, so fields with pins take single passes)
@@ -697,6 +705,7 @@ float* run_substeps_tma(float* a, float* b, const FieldMaps& m, int a_index, con
 
 int substep_launches(const FieldMaps& m, const FieldStep& fs, const Pins* pins) {
     if (pins && pins->n) return 2 * fs.substeps;
+    if (!m.passes && resident_fits(fs)) return RESIDENT_LEAD + 1;
     if (m.ok && m.pair_nt) return fs.substeps / 2 + (fs.substeps & 1);
     return fs.substeps;
 }
@@ -725,10 +734,13 @@ void launch_substep(const float* in, float* out, const FieldStep& fs, cudaStream
                                                        fs.inv_decay, fs.bval);
 }
 
-float* run_substeps(float* a, float* b, const FieldStep& fs, cudaStream_t s, const Pins* pins) {
+float* run_substeps(float* a, float* b, const FieldStep& fs, olc_u32* status, cudaStream_t s, const Pins* pins) {
     float* cur = a;
     float* nxt = b;
+    const bool resident = status && !(pins && pins->n) && resident_fits(fs);
     for (int i = 0; i < fs.substeps; ++i) {
+        if (resident && i == RESIDENT_LEAD)
+            if (float* res = run_resident(cur, nxt, fs, fs.substeps - i, status, s)) return res;
         launch_substep(cur, nxt, fs, s);
         launch_pins(nxt, pins, s);
         float* t = cur;
@@ -738,18 +750,10 @@ float* run_substeps(float* a, float* b, const FieldStep& fs, cudaStream_t s, con
     return cur;
 }
 
-float* run_field_step(float* a, float* b, float* sink, const FieldStep& fs, cudaStream_t s, const Pins* pins) {
+float* run_field_step(float* a, float* b, float* sink, const FieldStep& fs, olc_u32* status, cudaStream_t s,
+                      const Pins* pins) {
     launch_sink(a, sink, fs, s);
-    float* cur = a;
-    float* nxt = b;
-    for (int i = 0; i < fs.substeps; ++i) {
-        launch_substep(cur, nxt, fs, s);
-        launch_pins(nxt, pins, s);
-        float* t = cur;
-        cur = nxt;
-        nxt = t;
-    }
-    return cur;
+    return run_substeps(a, b, fs, status, s, pins);
 }
 
 }  // namespace olc

@@ -127,10 +127,11 @@ struct Pins {
 void launch_pins(float* f, const Pins* pins, cudaStream_t s);
 void launch_substep(const float* in, float* out, const FieldStep& fs, cudaStream_t s);
 // Runs sink + S substeps starting from a; returns the buffer holding the result.
-float* run_field_step(float* a, float* b, float* sink, const FieldStep& fs, cudaStream_t s,
+float* run_field_step(float* a, float* b, float* sink, const FieldStep& fs, olc_u32* status, cudaStream_t s,
                       const Pins* pins = nullptr);
 // The S substeps alone.
-float* run_substeps(float* a, float* b, const FieldStep& fs, cudaStream_t s, const Pins* pins = nullptr);
+float* run_substeps(float* a, float* b, const FieldStep& fs, olc_u32* status, cudaStream_t s,
+                    const Pins* pins = nullptr);
 // TMA tile path (x extent must be a multiple of 4): tensor maps of both
 // buffers for the single-substep kernel and for the T-substep temporal block.
 struct FieldMaps {
@@ -142,6 +143,7 @@ struct FieldMaps {
     int pair_nt = 0, pair_ty = 0, pair_zl = 0;
     CUtensorMap pair[2];
     int keep = 0;  // planes [0, keep) kept L2-resident across substeps by eviction hints (0: none)
+    bool passes = false;  // the caller's tuning names a shape of the passes: no other kernel instead of them
 };
 // The TMA tensor maps of a FP32 field's two buffers for the (tile_y, tile_z)
 // tile; false when the tile is not compiled in or the field cannot be mapped
@@ -158,6 +160,11 @@ bool stencil_tile_known(int tile_y, int tile_z);
 // Runs fs.substeps substeps starting from a (buffer index a_index of m).
 float* run_substeps_tma(float* a, float* b, const FieldMaps& m, int a_index, const FieldStep& fs, olc_u32* status,
                         cudaStream_t s, const Pins* pins = nullptr);
+// All remaining substeps of a small FP32 field in one cooperative launch
+// (olc_resident.cu), after RESIDENT_LEAD ordinary ones.
+constexpr int RESIDENT_LEAD = 2;
+bool resident_fits(const FieldStep& fs);
+float* run_resident(float* in, float* other, const FieldStep& fs, int substeps, olc_u32* status, cudaStream_t s);
 bool encode_map_elems(CUtensorMap* map, void* base, const int dims[3], const cuuint32_t box[3], int elem_bytes);
 
 // 16-bit field storage (olc_field16.cu): fields stored as BF16 or FP16,

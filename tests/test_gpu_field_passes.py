@@ -1,0 +1,54 @@
+"""The field kernels that run several substeps per launch, against the CPU
+oracle at the sizes where they can go wrong: bit for bit, as every kernel that
+uses only separately rounded + - * / and the clamp."""
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle
+from oncolytica_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _diffuse(cuda, olc, dims, substeps, boundary, decay=0.03, tuning=None, with_sink=False, low=-0.3):
+    import torch
+
+    nx, ny, nz = dims
+    rng = np.random.default_rng(nx * 7 + ny * 3 + nz + substeps)
+    f = (rng.random((nz, ny, nx), dtype=np.float32) + np.float32(low)).astype(np.float32)
+    sink = None
+    if with_sink:
+        sink = np.where(rng.random(f.shape) < 0.1, rng.random(f.shape), 0.0).astype(np.float32)
+    dt = 0.15 * substeps
+    ref = oracle.diffuse(f, sink, dx=1.0, dt=dt, D=1.0, decay=decay, boundary=boundary, substeps=substeps)
+    fd = torch.from_numpy(f.copy()).to(cuda)
+    # the other buffer's contents are the caller's leftovers, signs and all
+    tmp = torch.from_numpy(rng.standard_normal(f.shape).astype(np.float32)).to(cuda)
+    sd = torch.from_numpy(sink.copy()).to(cuda) if with_sink else None
+    spec = _lib.OlcDiffusion(diffusion=1.0, decay=decay, boundary=boundary, substeps=substeps,
+                             has_sink=int(with_sink))
+    dims_c = (C.c_int32 * 3)(nx, ny, nz)
+    _lib.check(olc.olc_stage_diffuse_tuned(C.c_void_p(fd.data_ptr()), C.c_void_p(tmp.data_ptr()),
+                                           C.c_void_p(sd.data_ptr()) if with_sink else None, C.byref(dims_c), 1.0, dt,
+                                           C.byref(spec), C.byref(tuning) if tuning is not None else None, None))
+    np.testing.assert_array_equal(fd.cpu().numpy(), ref)
+
+
+# rows that are no multiple of four, tiles of one row or plane, tiles that hold
+# only a face, more tiles than rows, rows longer than a warp's lanes
+RESIDENT_DIMS = [(3, 3, 3), (5, 9, 50), (20, 20, 20), (33, 5, 47), (64, 61, 67), (96, 96, 96), (131, 40, 38),
+                 (255, 7, 9), (256, 24, 25), (7, 150, 149)]
+
+
+@pytest.mark.parametrize("substeps", [6, 7, 12])
+@pytest.mark.parametrize("dims", RESIDENT_DIMS)
+def test_resident_field_bit_exact(cuda, olc, dims, substeps):
+    """A small field's substeps in one launch (two ordinary ones first):
+    an odd and an even number of exchanges, a negative boundary value, an input
+    and a second buffer with negative values."""
+    _diffuse(cuda, olc, dims, substeps, boundary=-0.4 if substeps == 7 else 0.6,
+             decay=0.0 if substeps == 12 else 0.03, with_sink=substeps == 6)
