@@ -151,15 +151,17 @@ typedef struct {
 #define OLC_CONTACT_FLAT   0  /* one flat walk over each agent's listed non-empty Moore bins */
 #define OLC_CONTACT_NESTED 1  /* nested loops over the 27 Moore bins                       */
 typedef struct {
-    int32_t stencil_tile_y;   /* FP32 TMA substep tile: rows (8 or 16) ...             */
+    int32_t stencil_tile_y;   /* tile of an FP32 one-substep pass: rows (8 or 16) ...  */
     int32_t stencil_tile_z;   /* ... and planes; (y, z) in {(8,8), (16,8), (8,16), (16,4)} */
     int32_t contact_variant;  /* OLC_CONTACT_FLAT or OLC_CONTACT_NESTED */
     int32_t batch_tile_depth; /* planes per tile of the batched FP32 substep: 8, 16 or
                                  32 (members without their own, olc_set_batch_tile_depths) */
-    int32_t stencil_pair_threads; /* two FP32 substeps per pass (temporal blocking) with
-                                     CTAs of 128, 256, 512 or 1024 threads where the field's
-                                     rows fit one TMA box (x extent <= 256); 0 = one
-                                     substep per pass */
+    int32_t stencil_pair_threads; /* 128, 256, 512 or 1024 (one kernel serves all): two FP32
+                                     substeps per pass (temporal blocking) where the field
+                                     allows it (x extent a multiple of 4, at least 16 rows and
+                                     8 planes, boundary >= 0).  0 = the library's choice for
+                                     the field's size, or one substep per pass when a tile
+                                     other than (8, 8) or a kept slab is asked for */
     int32_t stencil_pair_planes;  /* planes per CTA of the two-substep pass; 0 = as few
                                      as keep the whole grid resident in one wave */
     int32_t stencil_l2_keep_pct;  /* one-substep passes over an FP32 field read and write

@@ -6,7 +6,7 @@ candidate on the caller's own workload with per-stage CUDA events
 
 * ``tune_engine(engine)``: the FP32 stencil tile (rows x planes of the TMA
   substep), whether FP32 fields take two substeps per pass (temporal
-  blocking, and the CTA size of that kernel), the share of an FP32 field's
+  blocking), the share of an FP32 field's
   planes kept in L2 by eviction hints, and the contact walk of a solo
   engine.  The engine's state is saved
   with ``state_dict()`` first and restored after, so tuning leaves the run
@@ -33,21 +33,22 @@ STENCIL_TILES = ((8, 8), (16, 8), (8, 16), (16, 4))
 CONTACT_VARIANTS = (_lib.OLC_CONTACT_FLAT, _lib.OLC_CONTACT_NESTED)
 CONTACT_NAMES = {_lib.OLC_CONTACT_FLAT: "flat", _lib.OLC_CONTACT_NESTED: "nested"}
 BATCH_DEPTHS = (8, 16, 32)
-# (threads per CTA, planes per CTA) of the two-substeps-per-pass kernel; (0, 0) = one substep per pass
-STENCIL_PAIRS = ((0, 0), (1024, 0), (512, 0), (256, 0), (128, 0))
+# (threads per CTA, planes per CTA) of the two-substeps-per-pass kernel, which serves every CTA size
+# alike; (0, 0) = the library's choice
+STENCIL_PAIRS = ((0, 0), (256, 0))
 # share of an FP32 field's planes kept in L2 across one-substep passes (eviction hints)
 L2_KEEP = (0, 30, 45, 60)
 DEFAULT = {"stencil_tile": (8, 8), "contact_variant": _lib.OLC_CONTACT_FLAT, "batch_tile_depth": 16,
            "stencil_pair": (0, 0), "l2_keep_pct": 0}
-VERSION = 3  # cache entries of earlier tuners lack choices; they are measured again
+VERSION = 4  # cache entries of earlier tuners lack choices; they are measured again
 
 
 def pair_applies(threads: int, dims) -> bool:
     """Whether the two-substep kernel with ``threads`` per CTA runs on a field
-    of ``dims`` (x, y, z): rows of at most 256 voxels, x a multiple of 4, and
-    at least three intermediate rows per CTA (olc_field.cu pair_rows)."""
-    nx = int(dims[0])
-    return threads == 0 or (8 <= nx <= 256 and nx % 4 == 0 and threads // (nx // 4) >= 3)
+    of ``dims`` (x, y, z; olc_march.cu make_march_plan)."""
+    nx, ny, nz = (int(d) for d in dims)
+    return threads == 0 or (nx % 4 == 0 and ny >= 16 and nz >= 8)
+
 
 CACHE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_cache", "tuning.json")
 _lock = threading.Lock()

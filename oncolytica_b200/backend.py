@@ -368,7 +368,7 @@ class CudaBackend:
         """Kernel shapes and variants (olc_set_tuning): the FP32 stencil tile
         (rows, planes), the contact walk, the batched tile depth,
         ``stencil_pair`` = (threads per CTA, planes per CTA) of the
-        two-substeps-per-pass kernel ((0, 0): one substep per pass), and the
+        two-substeps-per-pass kernel ((0, 0): the library's choice), and the
         share of an FP32 field's planes kept in L2 across substeps by
         eviction hints (``l2_keep_pct``, 0: none)."""
         t = _lib.OlcTuning(int(stencil_tile[0]), int(stencil_tile[1]), int(contact_variant), int(batch_tile_depth),

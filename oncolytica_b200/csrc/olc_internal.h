@@ -132,27 +132,33 @@ float* run_field_step(float* a, float* b, float* sink, const FieldStep& fs, olc_
 // The S substeps alone.
 float* run_substeps(float* a, float* b, const FieldStep& fs, olc_u32* status, cudaStream_t s,
                     const Pins* pins = nullptr);
+// Two substeps per pass by warps marching along z (olc_march.cu).
+struct MarchPlan {
+    int lx = 0;              // lanes per row, 0: the march does not apply
+    int w = 0;               // warps per CTA
+    int gx = 0, gy = 0, gz = 0;  // grid
+    int zl = 0;              // planes per warp
+};
+bool march_pays(const int dims[3]);
+bool make_march_plan(const int dims[3], float bval, int planes, MarchPlan* p, cuuint32_t box[3]);
+void launch_march(const MarchPlan& p, const CUtensorMap& map, float* out, const FieldStep& fs, olc_u32* status, int down,
+                  cudaStream_t s);
 // TMA tile path (x extent must be a multiple of 4): tensor maps of both
 // buffers for the single-substep kernel and for the T-substep temporal block.
 struct FieldMaps {
     bool ok = false;
     int VY = 8, VZ = 8;  // tile of k_substep_x4: rows and planes (a compiled shape)
     CUtensorMap vec[2];
-    // two substeps per pass (k_substep_pair): threads per CTA (0: off), output
-    // rows per CTA, planes per CTA (0: as many as fill one wave of CTAs)
-    int pair_nt = 0, pair_ty = 0, pair_zl = 0;
-    CUtensorMap pair[2];
+    MarchPlan march;     // two substeps per pass (lx 0: off)
+    CUtensorMap march_map[2];
     int keep = 0;  // planes [0, keep) kept L2-resident across substeps by eviction hints (0: none)
     bool passes = false;  // the caller's tuning names a shape of the passes: no other kernel instead of them
 };
 // The TMA tensor maps of a FP32 field's two buffers for the (tile_y, tile_z)
 // tile; false when the tile is not compiled in or the field cannot be mapped
 // (the plain kernel runs then).
-bool make_field_maps(FieldMaps* m, float* a, float* b, const int dims[3], int tile_y = 8, int tile_z = 8,
+bool make_field_maps(FieldMaps* m, float* a, float* b, const int dims[3], float bval, int tile_y = 8, int tile_z = 8,
                      int pair_threads = 0, int pair_planes = 0, int keep_pct = 0);
-// k_substep_pair's output rows per CTA of nt threads on a field (0: it does
-// not apply), and whether nt is a compiled CTA size (0 included: off).
-int pair_rows(int nt, const int dims[3]);
 bool pair_threads_known(int nt);
 // Kernel launches of run_substeps_tma for one field step.
 int substep_launches(const FieldMaps& m, const FieldStep& fs, const Pins* pins);

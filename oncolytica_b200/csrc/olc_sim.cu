@@ -1282,7 +1282,8 @@ int olc_bind_field_ex(OlcSim* s, int index, void* a_, void* b_, float* sink, flo
     s->fmaps[index].ok = false;
     s->fmaps16[index].ok = false;
     if (spec->substeps > 0 && !half)
-        make_field_maps(&s->fmaps[index], a, b, s->geom.chem_dims, s->tuning.stencil_tile_y, s->tuning.stencil_tile_z,
+        make_field_maps(&s->fmaps[index], a, b, s->geom.chem_dims, spec->boundary, s->tuning.stencil_tile_y,
+                        s->tuning.stencil_tile_z,
                         s->tuning.stencil_pair_threads, s->tuning.stencil_pair_planes, s->tuning.stencil_l2_keep_pct);
     if (spec->substeps > 0 && half && !make_field_maps16(&s->fmaps16[index], a, b, s->geom.chem_dims))
         return fail(s, OLC_ERR_ARG, "olc_bind_field_ex: TMA descriptors of the 16-bit field failed (16-byte aligned "
@@ -2481,7 +2482,7 @@ static int stage_diffuse(float* f, float* tmp, float* sink, const int32_t dims[3
     FieldMaps maps;
     olc_u32* status = stage_status_word();
     float* res;
-    if (status && make_field_maps(&maps, f, tmp, dims, t->stencil_tile_y, t->stencil_tile_z, t->stencil_pair_threads,
+    if (status && make_field_maps(&maps, f, tmp, dims, spec->boundary, t->stencil_tile_y, t->stencil_tile_z, t->stencil_pair_threads,
                                   t->stencil_pair_planes, t->stencil_l2_keep_pct)) {
         launch_sink(f, spec->has_sink ? sink : nullptr, fs, st);
         res = run_substeps_tma(f, tmp, maps, 0, fs, status, st);
@@ -2519,7 +2520,7 @@ int olc_stage_diffuse_pinned(float* f, float* tmp, float* sink, const int32_t di
     FieldMaps maps;
     olc_u32* status = stage_status_word();
     float* res;
-    if (status && make_field_maps(&maps, f, tmp, dims)) {
+    if (status && make_field_maps(&maps, f, tmp, dims, spec->boundary)) {
         launch_sink(f, spec->has_sink ? sink : nullptr, fs, st);
         res = run_substeps_tma(f, tmp, maps, 0, fs, status, st, &pins);
     } else {
@@ -2719,7 +2720,8 @@ int olc_set_tuning(OlcSim* s, const OlcTuning* t) {
     if (!s->n_sims) {
         for (olc_u32 f = 0; f < s->caps.n_fields; ++f) {
             if (!s->field_bound[f] || s->fstep[f].storage != OLC_FIELD_F32 || s->fstep[f].substeps == 0) continue;
-            make_field_maps(&s->fmaps[f], s->field[0][f], s->field[1][f], s->geom.chem_dims, t->stencil_tile_y,
+            make_field_maps(&s->fmaps[f], s->field[0][f], s->field[1][f], s->geom.chem_dims, s->fspec[f].boundary,
+                            t->stencil_tile_y,
                             t->stencil_tile_z, t->stencil_pair_threads, t->stencil_pair_planes,
                             t->stencil_l2_keep_pct);
         }

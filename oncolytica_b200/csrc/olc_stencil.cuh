@@ -81,6 +81,28 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     return d;
 }
 
+// stencil_update4 with the x sums as scalars (their operands are shifted by one
+// voxel, so as pairs they would straddle register pairs) and every product
+// paired: the same operations and roundings.  A product that feeds a sum is
+// formed as a * b + (-0), which is the rounded product itself, the sign of a
+// zero included; the assembler cannot fuse that into the sum as long as it
+// does not see the -0, so nz2 comes from a kernel argument.  The decay factors
+// come as the pairs of the first and last two voxels (idl, idr), and the lower
+// bounds of the first and the last voxel as lo_l and lo_r (0 but for faces).
+__device__ __forceinline__ float4 stencil_update4f(float xl, float xr, const float4& c, const float4& ym,
+                                                   const float4& yp, const float4& zm, const float4& zp, f32x2 r2,
+                                                   f32x2 idl, f32x2 idr, float lo_l, float lo_r, f32x2 nz2) {
+    const f32x2 six = pk2(6.0f, 6.0f);
+    const f32x2 c0 = pk2(c.x, c.y), c1 = pk2(c.z, c.w);
+    const f32x2 x0 = pk2(__fadd_rn(xl, c.y), __fadd_rn(c.x, c.z)), x1 = pk2(__fadd_rn(c.y, c.w), __fadd_rn(c.z, xr));
+    const f32x2 s0 = add2(add2(x0, add2(pk2(ym.x, ym.y), pk2(yp.x, yp.y))), add2(pk2(zm.x, zm.y), pk2(zp.x, zp.y)));
+    const f32x2 s1 = add2(add2(x1, add2(pk2(ym.z, ym.w), pk2(yp.z, yp.w))), add2(pk2(zm.z, zm.w), pk2(zp.z, zp.w)));
+    const f32x2 u0 = add2(c0, fma2(r2, sub2(s0, fma2(six, c0, nz2)), nz2));
+    const f32x2 u1 = add2(c1, fma2(r2, sub2(s1, fma2(six, c1, nz2)), nz2));
+    const float2 a = upk2(mul2(u0, idl)), b = upk2(mul2(u1, idr));
+    return make_float4(fmaxf(a.x, lo_l), fmaxf(a.y, 0.0f), fmaxf(b.x, 0.0f), fmaxf(b.y, lo_r));
+}
+
 // The update of the 16-bit field storages: the same sums, with the two
 // products fused into their sums (one rounding each):
 //   u = fma(r, fma(-6, c, s), c),   out = max(u * inv_decay, 0)

@@ -52,3 +52,28 @@ def test_resident_field_bit_exact(cuda, olc, dims, substeps):
     and a second buffer with negative values."""
     _diffuse(cuda, olc, dims, substeps, boundary=-0.4 if substeps == 7 else 0.6,
              decay=0.0 if substeps == 12 else 0.03, with_sink=substeps == 6)
+
+
+# one and several tiles along x and y, last tiles that overlap the one before,
+# the smallest rows and planes the kernel takes, one plane per chunk and more
+MARCH_DIMS = [(64, 16, 8), (68, 33, 9), (128, 32, 8), (132, 34, 11), (256, 62, 13), (260, 40, 20), (300, 17, 70),
+              (4, 64, 9), (516, 65, 8)]
+
+
+@pytest.mark.parametrize("planes", [0, 1, 5])
+@pytest.mark.parametrize("substeps", [2, 5])
+@pytest.mark.parametrize("dims", MARCH_DIMS)
+def test_two_substeps_per_pass_bit_exact(cuda, olc, dims, substeps, planes):
+    """Two substeps per pass, up and down z, with the chunk lengths that divide
+    the planes and those that do not; boundary values at and above 0."""
+    tuning = _lib.OlcTuning(8, 8, 0, 16, 256, planes, 0)
+    _diffuse(cuda, olc, dims, substeps, boundary=0.0 if planes == 1 else 0.6, decay=0.03 if planes else 0.0,
+             tuning=tuning)
+
+
+def test_two_substeps_per_pass_leave_negative_boundaries_to_single_passes(cuda, olc):
+    _diffuse(cuda, olc, (64, 40, 20), 4, boundary=-0.25, tuning=_lib.OlcTuning(8, 8, 0, 16, 256, 0, 0))
+
+
+def test_large_field_takes_two_substeps_per_pass_by_itself(cuda, olc):
+    _diffuse(cuda, olc, (256, 130, 140), 7, boundary=0.5)
