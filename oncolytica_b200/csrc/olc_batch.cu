@@ -441,15 +441,40 @@ __global__ void __launch_bounds__(128) k_reduce_field_batch16(const uint4* __res
     const int z0 = (int)t.w * BT_Z;
     double sum = 0.0, mn = 1e300, mx = 0.0;
     if (x0 < nx && y < ny) {
+        // four voxels per 8- and 16-byte load (batched grids have x extents and
+        // offsets that are multiples of 4), four planes in flight; the extremes
+        // in FP32, which is exact
         const int z1 = min(z0 + BT_Z, nz);
-        for (int z = z0; z < z1; ++z)
-            for (int x = x0; x < x0 + 4; ++x) {
-                const size_t v = ((size_t)z * ny + y) * nx + x;
-                const double val = (double)phys_with_residual<ST, EN>(f[v], cp[v], ek);
-                sum += val;
-                mn = fmin(mn, val);
-                mx = fmax(mx, val);
+        float lo = __int_as_float(0x7f800000), hi = 0.0f;
+        const size_t sz = (size_t)nx * ny;
+        const size_t v0 = ((size_t)z0 * ny + y) * nx + x0;
+        if (((nx & 3) | (int)(d.field_off & 3)) == 0 &&
+            ((reinterpret_cast<uintptr_t>(f) & 7u) | (reinterpret_cast<uintptr_t>(cp) & 15u)) == 0) {
+#pragma unroll 4
+            for (int z = z0; z < z1; ++z) {
+                const size_t v = v0 + (size_t)(z - z0) * sz;
+                const uint2 h = __ldg(reinterpret_cast<const uint2*>(f + v));
+                const float4 c = __ldg(reinterpret_cast<const float4*>(cp + v));
+                const float p0 = phys_with_residual<ST, EN>((unsigned short)(h.x & 0xffffu), c.x, ek);
+                const float p1 = phys_with_residual<ST, EN>((unsigned short)(h.x >> 16), c.y, ek);
+                const float p2 = phys_with_residual<ST, EN>((unsigned short)(h.y & 0xffffu), c.z, ek);
+                const float p3 = phys_with_residual<ST, EN>((unsigned short)(h.y >> 16), c.w, ek);
+                sum += ((double)p0 + (double)p1) + ((double)p2 + (double)p3);
+                lo = fminf(lo, fminf(fminf(p0, p1), fminf(p2, p3)));
+                hi = fmaxf(hi, fmaxf(fmaxf(p0, p1), fmaxf(p2, p3)));
             }
+        } else {
+            for (int z = z0; z < z1; ++z)
+                for (int x = x0; x < x0 + 4 && x < nx; ++x) {
+                    const size_t v = ((size_t)z * ny + y) * nx + x;
+                    const float p = phys_with_residual<ST, EN>(f[v], cp[v], ek);
+                    sum += (double)p;
+                    lo = fminf(lo, p);
+                    hi = fmaxf(hi, p);
+                }
+        }
+        mn = fmin(mn, (double)lo);
+        mx = fmax(mx, (double)hi);
     }
     for (int o = 16; o > 0; o >>= 1) {
         sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -509,45 +534,114 @@ __device__ __forceinline__ void atomic_min_nonneg_b(double* p, double v) {
     atomicMin(reinterpret_cast<unsigned long long*>(p), (unsigned long long)__double_as_longlong(v));
 }
 
-// Per-simulation agent reductions (the solo k_reduce_agents per row, with the
-// row's simulation choosing the output record, centre and bin width).
-__global__ void __launch_bounds__(256) k_reduce_agents_batch(const float* __restrict__ x, const float* __restrict__ y,
-                                                             const float* __restrict__ z, const int* __restrict__ state,
-                                                             const olc_u32* __restrict__ sim,
-                                                             const unsigned char* __restrict__ life,
-                                                             const olc_u32* counters,
-                                                             const OlcSimDesc* __restrict__ sims, OlcReductions* out) {
+// Per-simulation agent reductions (k_reduce_agents's values, the row's
+// simulation choosing the output record, centre and bin width).
+//
+// One atomic per row and value serialised on the few records (285,000 agents of
+// 16 members: 0.6 ms).  Rows of a simulation are contiguous after the sort, so
+// each warp takes a run of RAB_ROWS consecutive rows, sums the simulation at
+// hand in registers (the histograms in its own shared-memory words) and adds to
+// the record only when the simulation changes and at the end of the run.
+constexpr olc_u32 RAB_ROWS = 512;
+constexpr int RAB_WARPS = 8;
+
+__global__ void __launch_bounds__(32 * RAB_WARPS) k_reduce_agents_batch(
+    const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ z, const int* __restrict__ state,
+    const olc_u32* __restrict__ sim, const unsigned char* __restrict__ life, const olc_u32* counters,
+    const OlcSimDesc* __restrict__ sims, OlcReductions* out) {
+    __shared__ olc_u32 s_hist[RAB_WARPS][OLC_RADIAL_BINS + OLC_STATE_BINS];
+    constexpr olc_u32 NONE = 0xffffffffu;
     const olc_u32 n = olc_total_rows(counters);
-    for (olc_u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (life[i]) continue;
-        const olc_u32 s = sim[i];
-        const OlcSimDesc& d = sims[s];
-        OlcReductions* o = out + s;
-        const float px = x[i], py = y[i], pz = z[i];
-        atomicAdd(&o->n_live, 1u);
-        atomicAdd(&o->sum_pos[0], (double)px);
-        atomicAdd(&o->sum_pos[1], (double)py);
-        atomicAdd(&o->sum_pos[2], (double)pz);
-        const double dx = (double)px - (double)d.center[0], dy = (double)py - (double)d.center[1],
-                     dz = (double)pz - (double)d.center[2];
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        atomicAdd(&o->sum_r2, r2);
-        const double r = sqrt(r2);
-        atomic_max_nonneg_b(&o->max_r, r);
-        int b = (int)(r / (double)(d.bin_width > 0.0f ? d.bin_width : 1.0f));
-        if (b >= OLC_RADIAL_BINS) b = OLC_RADIAL_BINS - 1;
-        atomicAdd(&o->radial_hist[b], 1u);
-        if (state) {
-            const int st = state[i];
-            if (st >= 0 && st < OLC_STATE_BINS) atomicAdd(&o->state_counts[st], 1u);
+    const int lane = threadIdx.x & 31;
+    olc_u32* hist = s_hist[threadIdx.x >> 5];
+    for (int k = lane; k < OLC_RADIAL_BINS + OLC_STATE_BINS; k += 32) hist[k] = 0u;
+    __syncwarp();
+    const olc_u32 warps = gridDim.x * RAB_WARPS, warp = blockIdx.x * RAB_WARPS + (threadIdx.x >> 5);
+    olc_u32 cur = NONE, live = 0;  // the simulation at hand (the same in every lane)
+    double sx = 0.0, sy = 0.0, sz = 0.0, sr2 = 0.0, mr = 0.0, cx = 0.0, cy = 0.0, cz = 0.0, bw = 1.0;
+    auto flush = [&]() {
+        if (cur == NONE) return;
+        OlcReductions* o = out + cur;
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1) {
+            sx += __shfl_xor_sync(0xffffffffu, sx, k);
+            sy += __shfl_xor_sync(0xffffffffu, sy, k);
+            sz += __shfl_xor_sync(0xffffffffu, sz, k);
+            sr2 += __shfl_xor_sync(0xffffffffu, sr2, k);
+            mr = fmax(mr, __shfl_xor_sync(0xffffffffu, mr, k));
+        }
+        live = __reduce_add_sync(0xffffffffu, live);
+        if (lane == 0 && live) {
+            atomicAdd(&o->n_live, live);
+            atomicAdd(&o->sum_pos[0], sx);
+            atomicAdd(&o->sum_pos[1], sy);
+            atomicAdd(&o->sum_pos[2], sz);
+            atomicAdd(&o->sum_r2, sr2);
+            atomic_max_nonneg_b(&o->max_r, mr);
+        }
+        __syncwarp();
+        for (int k = lane; k < OLC_RADIAL_BINS + OLC_STATE_BINS; k += 32) {
+            const olc_u32 v = hist[k];
+            if (v) atomicAdd(k < OLC_RADIAL_BINS ? &o->radial_hist[k] : &o->state_counts[k - OLC_RADIAL_BINS], v);
+            hist[k] = 0u;
+        }
+        __syncwarp();
+        sx = sy = sz = sr2 = mr = 0.0;
+        live = 0;
+    };
+    for (olc_u64 first = (olc_u64)warp * RAB_ROWS; first < n; first += (olc_u64)warps * RAB_ROWS) {
+        const olc_u32 last = (olc_u32)(first + RAB_ROWS < n ? first + RAB_ROWS : n);
+        for (olc_u32 base = (olc_u32)first; base < last; base += 32) {
+            const olc_u32 i = base + lane;
+            const bool on = i < last && life[i < last ? i : base] == 0;
+            const olc_u32 s = on ? sim[i] : NONE;
+            const float px = on ? x[i] : 0.0f, py = on ? y[i] : 0.0f, pz = on ? z[i] : 0.0f;
+            const int st = on && state ? state[i] : -1;
+            // the simulations among the 32 rows, one by one (nearly always one)
+            olc_u32 left = __ballot_sync(0xffffffffu, on);
+            while (left) {
+                const olc_u32 m = __shfl_sync(0xffffffffu, s, __ffs(left) - 1);
+                if (m != cur) {
+                    flush();
+                    cur = m;
+                    const OlcSimDesc& d = sims[m];
+                    cx = (double)d.center[0];
+                    cy = (double)d.center[1];
+                    cz = (double)d.center[2];
+                    bw = (double)(d.bin_width > 0.0f ? d.bin_width : 1.0f);
+                }
+                const bool mine = s == m;
+                left &= ~__ballot_sync(0xffffffffu, mine);
+                int b = -1;
+                if (mine) {
+                    ++live;
+                    sx += (double)px;
+                    sy += (double)py;
+                    sz += (double)pz;
+                    const double dx = (double)px - cx, dy = (double)py - cy, dz = (double)pz - cz;
+                    const double r2 = dx * dx + dy * dy + dz * dz;
+                    sr2 += r2;
+                    const double r = sqrt(r2);
+                    mr = fmax(mr, r);
+                    b = (int)(r / bw);
+                    if (b >= OLC_RADIAL_BINS) b = OLC_RADIAL_BINS - 1;
+                }
+                olc_u32 peers = __match_any_sync(0xffffffffu, b);
+                if (b >= 0 && lane == __ffs(peers) - 1) atomicAdd(&hist[b], (olc_u32)__popc(peers));
+                const int c = mine && st >= 0 && st < OLC_STATE_BINS ? st : -1;
+                peers = __match_any_sync(0xffffffffu, c);
+                if (c >= 0 && lane == __ffs(peers) - 1) atomicAdd(&hist[OLC_RADIAL_BINS + c], (olc_u32)__popc(peers));
+                __syncwarp();
+            }
         }
     }
+    flush();
 }
 
 void launch_reduce_agents_batch(const BatchArgs& b, const ReduceArgs& a, const olc_u32* sim, const olc_u32* counters,
                                 olc_u32 n_cap, OlcReductions* out, cudaStream_t s) {
-    k_reduce_agents_batch<<<grid_cap(n_cap, 256, sm_blocks(4)), 256, 0, s>>>(a.x, a.y, a.z, a.state, sim, a.life,
-                                                                            counters, b.sims, out);
+    k_reduce_agents_batch<<<grid_cap(n_cap, RAB_ROWS * RAB_WARPS, sm_blocks(4)), 32 * RAB_WARPS, 0, s>>>(
+        a.x, a.y, a.z, a.state, sim, a.life, counters, b.sims, out);
 }
 
 // Field mass / min / max per simulation: one block per tile.
