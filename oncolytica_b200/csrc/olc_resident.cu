@@ -6,8 +6,8 @@
 // and 9.7 at 117 x 75 x 131, whose rows no tensor map describes).  Here each
 // CTA of a cooperative grid (one per SM) keeps a tile of full rows in shared
 // memory, and the CTAs exchange only the tiles' outer rows after each substep
-// (whole field steps of 79, 88 and 21 substeps: 235 -> 112 us, 452 -> 193,
-// 203 -> 120).
+// (whole field steps of 79, 88 and 21 substeps: 235 -> 93 us, 452 -> 165,
+// 203 -> 98).
 //
 // Exchange without flags, fences or barriers: a substep's results are never
 // negative (the clamp), so the sign bit of a published word is free and carries
@@ -30,145 +30,156 @@
 #include "olc_stencil.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace olc {
 
 namespace {
 
-constexpr int RING_ITEMS = 4;  // ring groups per thread, at most
+constexpr int RING_ITEMS = 4;  // ring groups per thread, or row chunks of 128 words per warp, at most
 
 struct ResidentArgs {
-    float* in;      // the field: substep input, and every second exchange
-    float* other;   // the other buffer: first exchange
+    void* in;       // the field: substep input, and every second exchange
+    void* other;    // the other buffer: first exchange
     int nx, ny, nz;
     int G;          // groups of four voxels per row
     int By, Bz;     // rows and planes of a tile
     int ty;         // tiles along y
-    int runs;       // z runs per column of a tile
+    int runs, L;    // z runs per column of a tile, planes per run
     int substeps;   // >= 1
     float r, inv_decay, bval;
+    float neg_zero;  // -0.0f, where the compiler does not see it (stencil_update4f)
     olc_u32* status;
 };
 
-__device__ __forceinline__ uint4 ld_relaxed4(const float* p) {
-    uint4 v;
-    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p)
-                 : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_relaxed4(float* p, uint4 v) {
-    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z),
-                 "r"(v.w)
-                 : "memory");
-}
-
-// Four voxels of a row at x (x + 3 may pass the row's end: those words read as
-// `fill` and are not written).
+// FP32 elements.  VEC: rows of whole, 16-byte aligned groups; else a row's last
+// group may pass its end (those words read as `fill` and are not written).
 template <bool VEC>
-__device__ __forceinline__ uint4 ld_group(const float* row, int x, int nx, olc_u32 fill) {
-    if (VEC) return ld_relaxed4(row + x);
-    const olc_u32* w = reinterpret_cast<const olc_u32*>(row + x);
-    uint4 v = make_uint4(olc_ld_relaxed(w), fill, fill, fill);
-    if (x + 1 < nx) v.y = olc_ld_relaxed(w + 1);
-    if (x + 2 < nx) v.z = olc_ld_relaxed(w + 2);
-    if (x + 3 < nx) v.w = olc_ld_relaxed(w + 3);
-    return v;
-}
-template <bool VEC>
-__device__ __forceinline__ void st_group(float* row, int x, int nx, uint4 v) {
-    if (VEC) {
-        st_relaxed4(row + x, v);
-        return;
+struct ResidentF32 {
+    typedef uint4 Raw;
+    static constexpr bool GROUPS = VEC;  // the ring is read by groups (else by words)
+    static __device__ __forceinline__ Raw load(const void* f, olc_u32 v, int left, olc_u32 fill) {
+        const olc_u32* w = static_cast<const olc_u32*>(f) + v;
+        uint4 q = make_uint4(0u, fill, fill, fill);
+        if (VEC) {
+            asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w)
+                         : "l"(w));
+            return q;
+        }
+        q.x = olc_ld_relaxed(w);
+        if (left > 1) q.y = olc_ld_relaxed(w + 1);
+        if (left > 2) q.z = olc_ld_relaxed(w + 2);
+        if (left > 3) q.w = olc_ld_relaxed(w + 3);
+        return q;
     }
-    olc_u32* w = reinterpret_cast<olc_u32*>(row + x);
-    olc_st_relaxed(w, v.x);
-    if (x + 1 < nx) olc_st_relaxed(w + 1, v.y);
-    if (x + 2 < nx) olc_st_relaxed(w + 2, v.z);
-    if (x + 3 < nx) olc_st_relaxed(w + 3, v.w);
-}
+    static __device__ __forceinline__ void store(void* f, olc_u32 v, int left, Raw q) {
+        olc_u32* w = static_cast<olc_u32*>(f) + v;
+        if (VEC) {
+            asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(w), "r"(q.x), "r"(q.y), "r"(q.z),
+                         "r"(q.w));
+            return;
+        }
+        olc_st_relaxed(w, q.x);
+        if (left > 1) olc_st_relaxed(w + 1, q.y);
+        if (left > 2) olc_st_relaxed(w + 2, q.z);
+        if (left > 3) olc_st_relaxed(w + 3, q.w);
+    }
+    static constexpr olc_u32 PHASE = 0x80000000u;
+    static __device__ __forceinline__ olc_u32 load_word(const void* f, olc_u32 v) {
+        return olc_ld_relaxed(static_cast<const olc_u32*>(f) + v);
+    }
+    static __device__ __forceinline__ float word(olc_u32 w) { return __uint_as_float(w & 0x7fffffffu); }
+    static __device__ __forceinline__ bool ready(Raw q, olc_u32 phase) {
+        return (((q.x ^ phase) | (q.y ^ phase) | (q.z ^ phase) | (q.w ^ phase)) & PHASE) == 0u;
+    }
+    static __device__ __forceinline__ float4 value(Raw q) {
+        return make_float4(__uint_as_float(q.x & 0x7fffffffu), __uint_as_float(q.y & 0x7fffffffu),
+                           __uint_as_float(q.z & 0x7fffffffu), __uint_as_float(q.w & 0x7fffffffu));
+    }
+    static __device__ __forceinline__ Raw bits(float4 v, olc_u32 phase) {
+        return make_uint4(__float_as_uint(v.x) | phase, __float_as_uint(v.y) | phase, __float_as_uint(v.z) | phase,
+                          __float_as_uint(v.w) | phase);
+    }
+};
 
-__device__ __forceinline__ float4 as_f4(uint4 v) {
-    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+__device__ __forceinline__ float4 lds4(olc_u32 p) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(p));
+    return v;
 }
-__device__ __forceinline__ uint4 with_phase(float4 v, olc_u32 phase) {
-    return make_uint4((__float_as_uint(v.x) & 0x7fffffffu) | phase, (__float_as_uint(v.y) & 0x7fffffffu) | phase,
-                      (__float_as_uint(v.z) & 0x7fffffffu) | phase, (__float_as_uint(v.w) & 0x7fffffffu) | phase);
+__device__ __forceinline__ void sts4(olc_u32 p, float4 v) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w));
 }
 
 // One tile per CTA; a thread owns up to K consecutive planes of four voxels of
 // one row, in registers, and shares them with its neighbours through shared
-// memory (two copies of the tile and its ring of one row and one plane).
-template <int K, int NT, bool VEC>
+// memory (two copies of the tile and its ring of one row and one plane).  What
+// bounds it is latency (the exchange, about 0.8 us) and, on larger tiles,
+// instruction issue: the threads' addresses, faces and publications are worked
+// out once, before the substeps.
+template <int K, int NT, int RI, bool WRAP, class E>
 __global__ void __launch_bounds__(NT, 1) k_resident(const ResidentArgs a) {
     extern __shared__ __align__(16) float s_tile[];
     const int P = a.G * 4;                 // row pitch
-    const int Y2 = a.By + 2;               // rows held per plane, ring included
-    const int plane = Y2 * P;
+    const int plane = (a.By + 2) * P;
     const int copy = (a.Bz + 2) * plane;
     const int y0 = (blockIdx.x % a.ty) * a.By, z0 = (blockIdx.x / a.ty) * a.Bz;
     const int rows = min(a.By, a.ny - y0), planes = min(a.Bz, a.nz - z0);
-    const size_t sy = (size_t)a.nx, sz = (size_t)a.nx * a.ny;
+    const olc_u32 sy = (olc_u32)a.nx, sz = (olc_u32)a.nx * (olc_u32)a.ny;
     const int tid = threadIdx.x, lane = tid & 31;
+    const float bval = a.bval;
+    const float4 b4 = make_float4(bval, bval, bval, bval);
 
-    // this thread's column
+    // this thread's column of the tile; threads without one work on some other
+    // column's place and keep nothing
     const int per_run = a.G * a.By;
-    const int run = tid / per_run, col = tid - run * per_run;
+    const int run = min(tid / per_run, a.runs - 1), col = tid % per_run;
     const int ry = col / a.G, g = col - ry * a.G;
-    const int kz0 = run * K;
-    const int kn = (run < a.runs && ry < rows) ? min(K, planes - kz0) : 0;  // planes owned (<= 0: none)
-    const int x = 4 * g, y = y0 + ry;
-    const bool y_face = y == 0 || y >= a.ny - 1;
-    const int xe = a.nx - 1 - x;  // element of the row's last voxel, when within 0..3
-    float4 c[K];
-    const float4 b4 = make_float4(a.bval, a.bval, a.bval, a.bval);
-
-    // the ring's groups are dealt to the threads: rows below and above the
-    // tile (planes x 2), then planes below and above (rows x 2)
-    const int ring_rows = 2 * planes + 2 * rows;
-    const int ring_items = ring_rows * a.G;
-
-    // A ring group is read only where it and the own voxels next to it are
-    // inside the grid's faces (elsewhere bval stands in, and only face voxels
-    // see it), so two tiles always read each other or neither does.
-    int ring_so[RING_ITEMS], ring_gx[RING_ITEMS];  // place in shared memory (< 0: nothing to read), x
-    olc_u32 ring_go[RING_ITEMS];                   // first voxel of its row in the grid
-    auto interior = [&](int yy, int zz) {
-        const int Y = y0 + yy, Z = z0 + zz;
-        return Y > 0 && Y < a.ny - 1 && Z > 0 && Z < a.nz - 1;
-    };
-    auto fix_x = [&](float4 v, int gx) {
-        if (gx == 0) v.x = a.bval;
-        const int e = a.nx - 1 - gx;
-        if (e <= 0) v.x = a.bval;
-        if (e <= 1) v.y = a.bval;
-        if (e <= 2) v.z = a.bval;
-        if (e <= 3) v.w = a.bval;
-        return v;
-    };
-
-    // own voxels and the ring of the launch's input; the ring's face groups in both copies
+    const int kz0 = run * a.L;
+    const int x = 4 * g, y = y0 + ry, left = a.nx - x;
+    const bool has = tid < per_run * a.runs && ry < rows;
+    const int kn = min(a.L, planes - kz0);  // planes of the run (the last run may have fewer, or none)
     const int own = (kz0 + 1) * plane + (ry + 1) * P + x;
+    const olc_u32 vox = (olc_u32)(z0 + kz0) * sz + (olc_u32)y * sy + (olc_u32)x;
+    // bit k: plane k is computed here; is published after each substep
+    olc_u32 work = 0, publish = 0;
+    for (int k = 0; k < kn; ++k) {
+        const int z = z0 + kz0 + k;
+        const bool inner = has && y > 0 && y < a.ny - 1 && z > 0 && z < a.nz - 1;
+        work |= inner ? 1u << k : 0u;
+        publish |= inner && (ry == 0 || ry == rows - 1 || kz0 + k == 0 || kz0 + k == planes - 1) ? 1u << k : 0u;
+    }
+    // x faces (and what lies beyond a row's end): a factor 0 and a lower bound
+    // bval in the clamp that every voxel has
+    const bool f0 = x == 0 || left <= 1, f1 = left <= 2, f2 = left <= 3, f3 = left <= 4;
+    const f32x2 idl = pk2(f0 ? 0.0f : a.inv_decay, f1 ? 0.0f : a.inv_decay);
+    const f32x2 idr = pk2(f2 ? 0.0f : a.inv_decay, f3 ? 0.0f : a.inv_decay);
+    const float4 lo = make_float4(f0 ? bval : 0.0f, f1 ? bval : 0.0f, f2 ? bval : 0.0f, f3 ? bval : 0.0f);
+    const f32x2 r2 = pk2(a.r, a.r), nz2 = pk2(a.neg_zero, a.neg_zero);
+    // WRAP: rows go on in the next warp; its first and last lanes read their x
+    // neighbours from shared memory
+    const olc_u32 need_l = WRAP && lane == 0 && x > 0, need_r = WRAP && lane == 31 && left > 4;
+    const olc_u32 own_a = static_cast<olc_u32>(__cvta_generic_to_shared(s_tile + own));
+    const olc_u32 row_b = 4u * (olc_u32)P, plane_b = 4u * (olc_u32)plane;
+    const bool busy = __any_sync(0xffffffffu, work != 0u) != 0;
+
+    float4 c[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         c[k] = b4;
-        if (k < kn) {
-            const int z = z0 + kz0 + k;
-            if (!y_face && z > 0 && z < a.nz - 1)
-                c[k] = fix_x(as_f4(ld_group<VEC>(a.in + (size_t)z * sz + (size_t)y * sy, x, a.nx, 0u)), x);
+        if (k < kn && has) {
+            if (work >> k & 1u) c[k] = E::value(E::load(a.in, vox + (olc_u32)k * sz, left, 0u));
             *reinterpret_cast<float4*>(s_tile + own + k * plane) = c[k];
+            *reinterpret_cast<float4*>(s_tile + copy + own + k * plane) = c[k];
         }
     }
-#pragma unroll
-    for (int t = 0; t < RING_ITEMS; ++t) {
-        const int i = tid + t * NT;
-        ring_so[t] = -1;
-        ring_gx[t] = 0;
-        ring_go[t] = 0u;
-        if (i >= ring_items) continue;
-        const int rr = i / a.G;
-        const int gx = 4 * (i - rr * a.G);
+    // The ring: rows below and above the tile (planes x 2), then planes below and
+    // above (rows x 2).  A ring row is read only where it and the own row next to
+    // it are inside the grid's faces (elsewhere bval stands in, and only face
+    // voxels see it), so two tiles always read each other or neither does.
+    const int ring_rows = 2 * planes + 2 * rows;
+    auto ring_row = [&](int rr, int& so, olc_u32& go) {
         int yy, zz, iy, iz;
         if (rr < 2 * planes) {
             iz = zz = rr >> 1;
@@ -180,100 +191,155 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const ResidentArgs a) {
             zz = (q & 1) ? planes : -1;
             iz = (q & 1) ? planes - 1 : 0;
         }
-        const int so = (zz + 1) * plane + (yy + 1) * P + gx;
-        float4 v = b4;
-        if (interior(yy, zz) && interior(iy, iz)) {
-            ring_so[t] = so;
-            ring_gx[t] = gx;
-            ring_go[t] = (olc_u32)((size_t)(z0 + zz) * sz + (size_t)(y0 + yy) * sy);
-            v = fix_x(as_f4(ld_group<VEC>(a.in + ring_go[t], gx, a.nx, 0u)), gx);
-        } else {
-            *reinterpret_cast<float4*>(s_tile + copy + so) = b4;
+        so = (zz + 1) * plane + (yy + 1) * P;
+        const int Y = y0 + yy, Z = z0 + zz;
+        go = (olc_u32)Z * sz + (olc_u32)Y * sy;
+        iy += y0;
+        iz += z0;
+        return Y > 0 && Y < a.ny - 1 && Z > 0 && Z < a.nz - 1 && iy > 0 && iy < a.ny - 1 && iz > 0 && iz < a.nz - 1;
+    };
+    // by groups: dealt to the threads once; by words: a row per warp
+    int ring_so[RI];        // place in shared memory
+    olc_u32 ring_go[RI];    // voxel
+    olc_u32 ring_mask = 0;  // bit t: item t is read (by words: bit 4 t + j its word 32 j)
+    if (E::GROUPS) {
+#pragma unroll
+        for (int t = 0; t < RI; ++t) {
+            const int i = tid + t * NT;
+            ring_so[t] = 0;
+            ring_go[t] = 0u;
+            if (i >= ring_rows * a.G) continue;
+            const int rr = i / a.G;
+            const int gx = 4 * (i - rr * a.G);
+            int so;
+            olc_u32 go;
+            float4 v = b4;
+            const bool read = ring_row(rr, so, go);
+            so += gx;
+            if (read) {
+                ring_mask |= 1u << t;
+                ring_so[t] = so;
+                ring_go[t] = go + (olc_u32)gx;
+                v = E::value(E::load(a.in, ring_go[t], 4, 0u));
+            } else {
+                *reinterpret_cast<float4*>(s_tile + copy + so) = b4;
+            }
+            *reinterpret_cast<float4*>(s_tile + so) = v;
         }
-        *reinterpret_cast<float4*>(s_tile + so) = v;
+    } else {
+        for (int rr = tid >> 5; rr < ring_rows; rr += NT / 32) {
+            int so;
+            olc_u32 go;
+            const bool read = ring_row(rr, so, go);
+            for (int xx = lane; xx < P; xx += 32) {
+                s_tile[so + xx] = read && xx < a.nx ? E::word(E::load_word(a.in, go + (olc_u32)xx)) : bval;
+                s_tile[copy + so + xx] = bval;
+            }
+        }
+        const int chunks = (a.nx + 127) / 128;  // of 128 words
+#pragma unroll
+        for (int t = 0; t < RI; ++t) {
+            const int i = (tid >> 5) + t * (NT / 32), rr = i / chunks;
+            ring_so[t] = 0;
+            ring_go[t] = 0u;
+            if (i >= ring_rows * chunks || !ring_row(rr, ring_so[t], ring_go[t])) continue;
+            const int xx = lane + 128 * (i - rr * chunks);
+            ring_so[t] += xx;
+            ring_go[t] += (olc_u32)xx;
+            for (int j = 0; j < 4; ++j) ring_mask |= xx + 32 * j < a.nx ? 1u << (4 * t + j) : 0u;
+        }
     }
     __syncthreads();
 
     bool gave_up = false;
+    olc_u32 spins = 0;
     for (int e = 0;; ++e) {
-        const float* cur = s_tile + (e & 1) * copy;
-        float* nxt = s_tile + ((e & 1) ^ 1) * copy;
+        const int from = (e & 1) * copy, to = copy - from;
         const bool last = e == a.substeps - 1;
-        float* out = (e & 1) ? a.in : a.other;
-        const olc_u32 phase = (e & 2) ? 0u : 0x80000000u;
+        void* out = (e & 1) ? a.in : a.other;
+        const olc_u32 phase = (e & 2) ? 0u : E::PHASE;
+        const olc_u32 publish_now = last ? 0u : publish;
+        spins = 0;
         // ---- one substep of the own column
-        float4 prev = b4;
-        if (kn > 0) prev = *reinterpret_cast<const float4*>(cur + own - plane);
+        if (busy) {
+            olc_u32 pc = own_a + 4u * (olc_u32)from;  // the plane's own group, and the groups around it
+            olc_u32 pm = pc - row_b, pp = pc + row_b, pz = pc + plane_b, pn = own_a + 4u * (olc_u32)to;
+            olc_u32 vo = vox;
+            float4 prev = lds4(pc - plane_b);
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const float* pc = cur + own + k * plane;
-            float xl = __shfl_up_sync(0xffffffffu, c[k].w, 1);
-            float xr = __shfl_down_sync(0xffffffffu, c[k].x, 1);
-            if (k < kn) {
-                // a warp's first and last lanes: the neighbour group is another warp's
-                if (lane == 0 && x > 0) xl = pc[-1];
-                if (lane == 31 && xe > 3) xr = pc[4];
-                const float4 ym = *reinterpret_cast<const float4*>(pc - P);
-                const float4 yp = *reinterpret_cast<const float4*>(pc + P);
-                float4 zp;
-                if (k + 1 < K && k + 1 < kn)
-                    zp = c[k + 1 < K ? k + 1 : k];
-                else
-                    zp = *reinterpret_cast<const float4*>(pc + plane);
-                const int z = z0 + kz0 + k;
-                float4 v = stencil_update4(xl, xr, c[k], ym, yp, prev, zp, a.r, a.inv_decay);
-                if (y_face || z == 0 || z == a.nz - 1) {
-                    v = b4;
-                } else {
-                    if (x == 0) v.x = a.bval;
-                    if (xe <= 3) {
-                        if (xe <= 0) v.x = a.bval;
-                        if (xe <= 1) v.y = a.bval;
-                        if (xe <= 2) v.z = a.bval;
-                        v.w = a.bval;
-                    }
+            for (int k = 0; k < K; ++k) {
+                if (k >= a.L) break;  // the same for every thread: lanes of one warp may belong to different runs
+                float xl = __shfl_up_sync(0xffffffffu, c[k].w, 1);
+                float xr = __shfl_down_sync(0xffffffffu, c[k].x, 1);
+                if (WRAP) {
+                    asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; @p ld.shared.f32 %0, [%1 + -4]; }"
+                                 : "+f"(xl) : "r"(pc), "r"(need_l));
+                    asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; @p ld.shared.f32 %0, [%1 + 16]; }"
+                                 : "+f"(xr) : "r"(pc), "r"(need_r));
                 }
-                if (last) {
-                    float* row = out + (size_t)z * sz + (size_t)y * sy;
-                    st_group<VEC>(row, x, a.nx, make_uint4(__float_as_uint(v.x), __float_as_uint(v.y),
-                                                           __float_as_uint(v.z), __float_as_uint(v.w)));
-                } else {
-                    *reinterpret_cast<float4*>(nxt + own + k * plane) = v;
-                    if (ry == 0 || ry == rows - 1 || kz0 + k == 0 || kz0 + k == planes - 1)
-                        st_group<VEC>(out + (size_t)z * sz + (size_t)y * sy, x, a.nx, with_phase(v, phase));
-                }
+                const float4 v = stencil_update4g(xl, xr, c[k], lds4(pm), lds4(pp), prev, lds4(pz), r2, idl, idr, lo, nz2);
                 prev = c[k];
-                c[k] = v;
+                if (work >> k & 1u) {
+                    c[k] = v;
+                    sts4(pn, v);
+                }
+                if (publish_now >> k & 1u) E::store(out, vo, left, E::bits(v, phase));
+                pc += plane_b;
+                pm += plane_b;
+                pp += plane_b;
+                pz += plane_b;
+                pn += plane_b;
+                vo += sz;
             }
         }
-        if (last) return;
-        // ---- the neighbours' outer rows
-        uint4 w[RING_ITEMS];
+        if (last) {
 #pragma unroll
-        for (int t = 0; t < RING_ITEMS; ++t)
-            if (ring_so[t] >= 0) w[t] = ld_group<VEC>(out + ring_go[t], ring_gx[t], a.nx, phase);
+            for (int k = 0; k < K; ++k)
+                if (k < kn && has) E::store(out, vox + (olc_u32)k * sz, left, E::bits(c[k], 0u));
+            return;
+        }
+        // ---- the neighbours' outer rows.  Few polls are in flight at a time: the
+        // tiles still computing would wait behind them.
+        auto wait_more = [&]() {
+            if (gave_up) return false;
+            if (++spins <= OLC_SPIN_LIMIT) return true;
+            atomicOr(a.status, OLC_ST_TIMEOUT);
+            gave_up = true;
+            return false;
+        };
+        if (E::GROUPS) {
+            typename E::Raw w[RI];
 #pragma unroll
-        for (int t = 0; t < RING_ITEMS; ++t) {
-            if (ring_so[t] < 0) continue;
-            olc_u32 spins = 0;
-            while (!gave_up &&
-                   (((w[t].x ^ phase) | (w[t].y ^ phase) | (w[t].z ^ phase) | (w[t].w ^ phase)) & 0x80000000u)) {
-                if (++spins > OLC_SPIN_LIMIT) {
-                    atomicOr(a.status, OLC_ST_TIMEOUT);
-                    gave_up = true;
-                }
-                w[t] = ld_group<VEC>(out + ring_go[t], ring_gx[t], a.nx, phase);
+            for (int t = 0; t < RI; ++t)
+                if (ring_mask >> t & 1u) w[t] = E::load(out, ring_go[t], 4, phase);
+#pragma unroll
+            for (int t = 0; t < RI; ++t) {
+                if (!(ring_mask >> t & 1u)) continue;
+                while (!E::ready(w[t], phase) && wait_more()) w[t] = E::load(out, ring_go[t], 4, phase);
+                *reinterpret_cast<float4*>(s_tile + to + ring_so[t]) = E::value(w[t]);
             }
-            const uint4 v = make_uint4(w[t].x & 0x7fffffffu, w[t].y & 0x7fffffffu, w[t].z & 0x7fffffffu,
-                                       w[t].w & 0x7fffffffu);
-            *reinterpret_cast<float4*>(nxt + ring_so[t]) = fix_x(as_f4(v), ring_gx[t]);
+        } else {
+            olc_u32 w[4 * RI];
+            olc_u32 missing = ring_mask;
+            while (missing) {
+#pragma unroll
+                for (int t = 0; t < 4 * RI; ++t)
+                    if (missing >> t & 1u) w[t] = E::load_word(out, ring_go[t >> 2] + 32u * (t & 3));
+                const bool more = wait_more();
+#pragma unroll
+                for (int t = 0; t < 4 * RI; ++t) {
+                    if (!(missing >> t & 1u) || (more && ((w[t] ^ phase) & E::PHASE))) continue;
+                    missing &= ~(1u << t);
+                    s_tile[to + ring_so[t >> 2] + 32 * (t & 3)] = E::word(w[t]);
+                }
+            }
         }
         __syncthreads();
     }
 }
 
 struct ResidentPlan {
-    int By = 0, Bz = 0, ty = 0, tz = 0, K = 0, NT = 0, runs = 0;
+    int By = 0, Bz = 0, ty = 0, tz = 0, K = 0, NT = 0, RI = 0, runs = 0, L = 0;
     size_t smem = 0;
 };
 
@@ -289,7 +355,7 @@ constexpr size_t RES_SMEM_MAX = 225 * 1024;
 // Tile of the field's rows and planes: at most one tile per SM, the least
 // arithmetic and exchange per tile (a ring row costs about as much as two
 // rows of arithmetic: it is published, polled and staged).
-bool make_resident_plan(const int dims[3], int sms, ResidentPlan* best) {
+bool make_resident_plan(const int dims[3], bool groups, int sms, ResidentPlan* best) {
     const int nx = dims[0], ny = dims[1], nz = dims[2];
     const int G = (nx + 3) / 4;
     double best_cost = 1e30;
@@ -299,15 +365,19 @@ bool make_resident_plan(const int dims[3], int sms, ResidentPlan* best) {
         const int tz_max = sms / ty;
         const int Bz = (nz + tz_max - 1) / tz_max;
         const int tz = (nz + Bz - 1) / Bz;
-        const size_t smem = 2 * (size_t)(By + 2) * (Bz + 2) * G * 16;
-        if (smem > RES_SMEM_MAX) continue;
         const int cols = G * By;
         for (int K = 1; K <= 8; K *= 2) {
             const int runs = (Bz + K - 1) / K;
             const int threads = cols * runs;
             if (threads > 512) continue;
-            const int nt = threads <= 256 ? 256 : 512;
-            if (2 * (By + Bz) * G > RING_ITEMS * nt) continue;
+            const int nt = K == 1 && threads <= 256 ? 256 : 512;
+            // ring groups per thread, or 128-word chunks of ring rows per warp
+            const int ring = 2 * (By + Bz) * (groups ? G : (nx + 127) / 128), takers = groups ? nt : nt / 32;
+            if (ring > RING_ITEMS * takers) continue;
+            // the last run's loop reads past the tile where it has fewer planes
+            const int L = (Bz + runs - 1) / runs;
+            const size_t smem = (size_t)(By + 2) * (2 * (Bz + 2) + runs * L - Bz) * G * 16;
+            if (smem > RES_SMEM_MAX) continue;
             const double cost = By * Bz + 4.0 * (By + Bz) + 0.5 * K;
             if (cost < best_cost) {
                 best_cost = cost;
@@ -317,7 +387,9 @@ bool make_resident_plan(const int dims[3], int sms, ResidentPlan* best) {
                 best->tz = tz;
                 best->K = K;
                 best->runs = runs;
+                best->L = L;
                 best->NT = nt;
+                best->RI = ring <= takers ? 1 : RING_ITEMS;
                 best->smem = smem;
             }
             break;  // fewer planes per thread fill the SM better
@@ -326,13 +398,14 @@ bool make_resident_plan(const int dims[3], int sms, ResidentPlan* best) {
     return best_cost < 1e30;
 }
 
-template <int K, int NT, bool VEC>
-cudaError_t launch_resident(const ResidentArgs& a, const ResidentPlan& p, cudaStream_t s) {
+template <int K, int NT, int RI, bool WRAP, class E>
+cudaError_t launch_resident_t(const ResidentArgs& a, const ResidentPlan& p, cudaStream_t s) {
     static int configured_mask = 0;  // per device (up to 32)
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 32 && !(configured_mask & (1 << dev))) {
-        cudaFuncSetAttribute(k_resident<K, NT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM_MAX);
+        cudaFuncSetAttribute(k_resident<K, NT, RI, WRAP, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)RES_SMEM_MAX);
         configured_mask |= 1 << dev;
     }
     cudaLaunchConfig_t cfg = {};
@@ -345,40 +418,46 @@ cudaError_t launch_resident(const ResidentArgs& a, const ResidentPlan& p, cudaSt
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_resident<K, NT, VEC>, a);
+    return cudaLaunchKernelEx(&cfg, k_resident<K, NT, RI, WRAP, E>, a);
 }
 
-template <bool VEC>
+template <int K, int NT, class E>
 cudaError_t launch_resident_k(const ResidentArgs& a, const ResidentPlan& p, cudaStream_t s) {
-#define OLC_RES_CASE(k, nt) \
-    if (p.K == k && p.NT == nt) return launch_resident<k, nt, VEC>(a, p, s);
-    OLC_RES_CASE(1, 256)
-    OLC_RES_CASE(1, 512)
-    OLC_RES_CASE(2, 256)
-    OLC_RES_CASE(2, 512)
-    OLC_RES_CASE(4, 256)
-    OLC_RES_CASE(4, 512)
-    OLC_RES_CASE(8, 256)
-    OLC_RES_CASE(8, 512)
-#undef OLC_RES_CASE
-    return cudaErrorInvalidValue;
+    if (!E::GROUPS) return launch_resident_t<K, NT, RING_ITEMS, true, E>(a, p, s);
+    const bool wrap = a.G > 32 || (32 % a.G) != 0;
+    if (p.RI == 1)
+        return wrap ? launch_resident_t<K, NT, 1, true, E>(a, p, s) : launch_resident_t<K, NT, 1, false, E>(a, p, s);
+    return wrap ? launch_resident_t<K, NT, RING_ITEMS, true, E>(a, p, s)
+                : launch_resident_t<K, NT, RING_ITEMS, false, E>(a, p, s);
+}
+
+template <class E>
+cudaError_t launch_resident(const ResidentArgs& a, const ResidentPlan& p, cudaStream_t s) {
+    if (p.NT == 256) return launch_resident_k<1, 256, E>(a, p, s);
+    if (p.K == 1) return launch_resident_k<1, 512, E>(a, p, s);
+    if (p.K == 2) return launch_resident_k<2, 512, E>(a, p, s);
+    if (p.K == 4) return launch_resident_k<4, 512, E>(a, p, s);
+    return launch_resident_k<8, 512, E>(a, p, s);
 }
 
 }  // namespace
 
 // Whether a field's substeps are worth the resident launch.
 bool resident_fits(const FieldStep& fs) {
-    if (fs.substeps < RESIDENT_LEAD + 4) return false;
+    // faces get their value as the clamp's lower bound, which needs bval >= +0
+    if (fs.substeps < RESIDENT_LEAD + 4 || !(fs.bval >= 0.0f) || std::signbit(fs.bval)) return false;
     ResidentPlan p;
-    return make_resident_plan(fs.dims, device_sms(), &p);
+    return make_resident_plan(fs.dims, (fs.dims[0] & 3) == 0, device_sms(), &p);
 }
 
 // `substeps` substeps from `in` (both buffers hold substep results: clear sign
 // bits); returns the buffer holding the result, or null when the launch was
 // not possible.
 float* run_resident(float* in, float* other, const FieldStep& fs, int substeps, olc_u32* status, cudaStream_t s) {
+    const bool vec =
+        (fs.dims[0] & 3) == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(other)) & 15u) == 0;
     ResidentPlan p;
-    if (substeps < 1 || !make_resident_plan(fs.dims, device_sms(), &p)) return nullptr;
+    if (substeps < 1 || !make_resident_plan(fs.dims, vec, device_sms(), &p)) return nullptr;
     ResidentArgs a;
     a.in = in;
     a.other = other;
@@ -390,13 +469,14 @@ float* run_resident(float* in, float* other, const FieldStep& fs, int substeps, 
     a.Bz = p.Bz;
     a.ty = p.ty;
     a.runs = p.runs;
+    a.L = p.L;
     a.substeps = substeps;
     a.r = fs.r;
     a.inv_decay = fs.inv_decay;
     a.bval = fs.bval;
+    a.neg_zero = -0.0f;
     a.status = status;
-    const bool vec = (a.nx & 3) == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(other)) & 15u) == 0;
-    const cudaError_t e = vec ? launch_resident_k<true>(a, p, s) : launch_resident_k<false>(a, p, s);
+    const cudaError_t e = vec ? launch_resident<ResidentF32<true>>(a, p, s) : launch_resident<ResidentF32<false>>(a, p, s);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return nullptr;

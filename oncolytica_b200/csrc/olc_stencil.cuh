@@ -89,9 +89,9 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 // does not see the -0, so nz2 comes from a kernel argument.  The decay factors
 // come as the pairs of the first and last two voxels (idl, idr), and the lower
 // bounds of the first and the last voxel as lo_l and lo_r (0 but for faces).
-__device__ __forceinline__ float4 stencil_update4f(float xl, float xr, const float4& c, const float4& ym,
+__device__ __forceinline__ float4 stencil_update4u(float xl, float xr, const float4& c, const float4& ym,
                                                    const float4& yp, const float4& zm, const float4& zp, f32x2 r2,
-                                                   f32x2 idl, f32x2 idr, float lo_l, float lo_r, f32x2 nz2) {
+                                                   f32x2 idl, f32x2 idr, f32x2 nz2) {
     const f32x2 six = pk2(6.0f, 6.0f);
     const f32x2 c0 = pk2(c.x, c.y), c1 = pk2(c.z, c.w);
     const f32x2 x0 = pk2(__fadd_rn(xl, c.y), __fadd_rn(c.x, c.z)), x1 = pk2(__fadd_rn(c.y, c.w), __fadd_rn(c.z, xr));
@@ -100,7 +100,21 @@ __device__ __forceinline__ float4 stencil_update4f(float xl, float xr, const flo
     const f32x2 u0 = add2(c0, fma2(r2, sub2(s0, fma2(six, c0, nz2)), nz2));
     const f32x2 u1 = add2(c1, fma2(r2, sub2(s1, fma2(six, c1, nz2)), nz2));
     const float2 a = upk2(mul2(u0, idl)), b = upk2(mul2(u1, idr));
-    return make_float4(fmaxf(a.x, lo_l), fmaxf(a.y, 0.0f), fmaxf(b.x, 0.0f), fmaxf(b.y, lo_r));
+    return make_float4(a.x, a.y, b.x, b.y);  // not yet clamped
+}
+__device__ __forceinline__ float4 stencil_update4f(float xl, float xr, const float4& c, const float4& ym,
+                                                   const float4& yp, const float4& zm, const float4& zp, f32x2 r2,
+                                                   f32x2 idl, f32x2 idr, float lo_l, float lo_r, f32x2 nz2) {
+    const float4 v = stencil_update4u(xl, xr, c, ym, yp, zm, zp, r2, idl, idr, nz2);
+    return make_float4(fmaxf(v.x, lo_l), fmaxf(v.y, 0.0f), fmaxf(v.z, 0.0f), fmaxf(v.w, lo_r));
+}
+
+// stencil_update4f with a lower bound for each voxel.
+__device__ __forceinline__ float4 stencil_update4g(float xl, float xr, const float4& c, const float4& ym,
+                                                   const float4& yp, const float4& zm, const float4& zp, f32x2 r2,
+                                                   f32x2 idl, f32x2 idr, const float4& lo, f32x2 nz2) {
+    const float4 v = stencil_update4u(xl, xr, c, ym, yp, zm, zp, r2, idl, idr, nz2);
+    return make_float4(fmaxf(v.x, lo.x), fmaxf(v.y, lo.y), fmaxf(v.z, lo.z), fmaxf(v.w, lo.w));
 }
 
 // The update of the 16-bit field storages: the same sums, with the two

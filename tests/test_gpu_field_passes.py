@@ -48,8 +48,8 @@ RESIDENT_DIMS = [(3, 3, 3), (5, 9, 50), (20, 20, 20), (33, 5, 47), (64, 61, 67),
 @pytest.mark.parametrize("dims", RESIDENT_DIMS)
 def test_resident_field_bit_exact(cuda, olc, dims, substeps):
     """A small field's substeps in one launch (two ordinary ones first):
-    an odd and an even number of exchanges, a negative boundary value, an input
-    and a second buffer with negative values."""
+    an odd and an even number of exchanges, a negative boundary value (left to
+    one launch per substep), an input and a second buffer with negative values."""
     _diffuse(cuda, olc, dims, substeps, boundary=-0.4 if substeps == 7 else 0.6,
              decay=0.0 if substeps == 12 else 0.03, with_sink=substeps == 6)
 
