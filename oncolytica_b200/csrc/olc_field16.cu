@@ -369,7 +369,12 @@ void* run_substeps16(void* a, void* b, const FieldMaps16& m, int a_index, const 
     bufs[a_index] = a;
     bufs[1 - a_index] = b;
     int cur = a_index;
+    const bool resident = resident_fits16(fs);
     for (int i = 0; i < fs.substeps; ++i) {
+        if (resident && i == RESIDENT_LEAD)
+            if (void* res = run_resident16(bufs[cur], bufs[1 - cur], fs, fs.substeps - i, status, step_ctr, step_host, i,
+                                           field, s))
+                return res;
         with_storage16(fs.storage, fs.encoding, [&](auto st, auto en) {
             launch_sub16<decltype(st)::value, decltype(en)::value>(m.map[cur], bufs[1 - cur], fs, status, i & 1,
                                                                    step_ctr, step_host, i, field, s);

@@ -166,11 +166,14 @@ bool stencil_tile_known(int tile_y, int tile_z);
 // Runs fs.substeps substeps starting from a (buffer index a_index of m).
 float* run_substeps_tma(float* a, float* b, const FieldMaps& m, int a_index, const FieldStep& fs, olc_u32* status,
                         cudaStream_t s, const Pins* pins = nullptr);
-// All remaining substeps of a small FP32 field in one cooperative launch
+// All remaining substeps of a small field in one cooperative launch
 // (olc_resident.cu), after RESIDENT_LEAD ordinary ones.
 constexpr int RESIDENT_LEAD = 2;
 bool resident_fits(const FieldStep& fs);
 float* run_resident(float* in, float* other, const FieldStep& fs, int substeps, olc_u32* status, cudaStream_t s);
+bool resident_fits16(const FieldStep& fs);
+void* run_resident16(void* in, void* other, const FieldStep& fs, int substeps, olc_u32* status, const olc_u32* step_ctr,
+                     olc_u32 step_host, int sub0, int field, cudaStream_t s);
 bool encode_map_elems(CUtensorMap* map, void* base, const int dims[3], const cuuint32_t box[3], int elem_bytes);
 
 // 16-bit field storage (olc_field16.cu): fields stored as BF16 or FP16,

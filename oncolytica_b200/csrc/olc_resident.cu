@@ -1,4 +1,4 @@
-// FP32 fields small enough to stay on chip: all the remaining substeps of a
+// Fields small enough to stay on chip: all the remaining substeps of a
 // field step in one launch.
 //
 // A substep of a small field is a fraction of a microsecond of arithmetic; as
@@ -24,10 +24,15 @@
 // All waits are bounded: a thread that gives up records OLC_ST_TIMEOUT and
 // polls no more, so the grid always ends.
 //
-// Per voxel the update is stencil_update4, so the result equals the
-// one-launch-per-substep kernels bit for bit.
+// Per voxel the update, and the rounding of 16-bit storage, are those of the
+// one-launch-per-substep kernels, so the results equal theirs bit for bit.
+// 16-bit fields keep FP32 working values on chip: each is decoded once per
+// substep instead of at each of its neighbours (3.25 times).  Their exchange
+// needs the element's sign bit too, which values and deficits leave clear;
+// three-offset elements use all their bits and are left to single passes.
 #include "olc_internal.h"
 #include "olc_stencil.cuh"
+#include "olc_store16.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -47,9 +52,16 @@ struct ResidentArgs {
     int ty;         // tiles along y
     int runs, L;    // z runs per column of a tile, planes per run
     int substeps;   // >= 1
-    float r, inv_decay, bval;
+    float r, inv_decay;
+    float bval;     // the boundary value
     float neg_zero;  // -0.0f, where the compiler does not see it (stencil_update4f)
     olc_u32* status;
+    // 16-bit storage: the deficits' decay term, and what salts
+    // the stochastic rounding (the step from step_ctr, else step_host)
+    float dec_sub;
+    const olc_u32* step_ctr;
+    olc_u32 step_host;
+    int sub0, field;
 };
 
 // FP32 elements.  VEC: rows of whole, 16-byte aligned groups; else a row's last
@@ -90,6 +102,27 @@ struct ResidentF32 {
         return olc_ld_relaxed(static_cast<const olc_u32*>(f) + v);
     }
     static __device__ __forceinline__ float word(olc_u32 w) { return __uint_as_float(w & 0x7fffffffu); }
+    static constexpr bool ROUNDS = false;
+    static __device__ __forceinline__ float face(float bval) { return bval; }
+    static __device__ __forceinline__ float4 round(float4 v, olc_u32, olc_u32) { return v; }
+    struct Update {
+        f32x2 r2, idl, idr, nz2;
+        float4 lo;
+        // f[e]: voxel e is a face (or lies beyond the row): a factor 0 and a
+        // lower bound bval in the clamp that every voxel has
+        __device__ __forceinline__ Update(const ResidentArgs& a, float bval, const bool (&f)[4]) {
+            r2 = pk2(a.r, a.r);
+            nz2 = pk2(a.neg_zero, a.neg_zero);
+            idl = pk2(f[0] ? 0.0f : a.inv_decay, f[1] ? 0.0f : a.inv_decay);
+            idr = pk2(f[2] ? 0.0f : a.inv_decay, f[3] ? 0.0f : a.inv_decay);
+            lo = make_float4(f[0] ? bval : 0.0f, f[1] ? bval : 0.0f, f[2] ? bval : 0.0f, f[3] ? bval : 0.0f);
+        }
+        __device__ __forceinline__ float4 operator()(float xl, float xr, const float4& c, const float4& ym,
+                                                     const float4& yp, const float4& zm, const float4& zp) const {
+            const float4 v = stencil_update4u(xl, xr, c, ym, yp, zm, zp, r2, idl, idr, nz2);
+            return make_float4(fmaxf(v.x, lo.x), fmaxf(v.y, lo.y), fmaxf(v.z, lo.z), fmaxf(v.w, lo.w));
+        }
+    };
     static __device__ __forceinline__ bool ready(Raw q, olc_u32 phase) {
         return (((q.x ^ phase) | (q.y ^ phase) | (q.z ^ phase) | (q.w ^ phase)) & PHASE) == 0u;
     }
@@ -101,6 +134,75 @@ struct ResidentF32 {
         return make_uint4(__float_as_uint(v.x) | phase, __float_as_uint(v.y) | phase, __float_as_uint(v.z) | phase,
                           __float_as_uint(v.w) | phase);
     }
+};
+
+// 16-bit elements holding values or deficits (rows are whole groups: the x
+// extent is a multiple of 8 and the buffers are 16-byte aligned).
+template <int ST, int EN>
+struct Resident16 {
+    static_assert(EN != OLC_ENC_OFFSET3, "three-offset elements have no free bit");
+    typedef uint2 Raw;
+    static constexpr bool GROUPS = true;
+    static constexpr olc_u32 PHASE = 0x80008000u;
+    static __device__ __forceinline__ Raw load(const void* f, olc_u32 v, int, olc_u32) {
+        uint2 q;
+        asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];"
+                     : "=r"(q.x), "=r"(q.y)
+                     : "l"(static_cast<const unsigned short*>(f) + v));
+        return q;
+    }
+    static __device__ __forceinline__ void store(void* f, olc_u32 v, int, Raw q) {
+        asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(static_cast<unsigned short*>(f) + v), "r"(q.x),
+                     "r"(q.y));
+    }
+    static __device__ __forceinline__ bool ready(Raw q, olc_u32 phase) {
+        return (((q.x ^ phase) | (q.y ^ phase)) & PHASE) == 0u;
+    }
+    static __device__ __forceinline__ float4 value(Raw q) {
+        const olc_u32 x = q.x & ~PHASE, y = q.y & ~PHASE;
+        return make_float4(Store16<ST>::to_f((unsigned short)(x & 0xffffu)), Store16<ST>::to_f((unsigned short)(x >> 16)),
+                           Store16<ST>::to_f((unsigned short)(y & 0xffffu)), Store16<ST>::to_f((unsigned short)(y >> 16)));
+    }
+    // v holds values that were rounded to storage: the conversion is exact
+    static __device__ __forceinline__ Raw bits(float4 v, olc_u32 phase) {
+        return make_uint2(pack2<ST>(v.x, v.y) | phase, pack2<ST>(v.z, v.w) | phase);
+    }
+    static __device__ __forceinline__ olc_u32 load_word(const void*, olc_u32) { return 0u; }
+    static __device__ __forceinline__ float word(olc_u32) { return 0.0f; }
+    static constexpr bool ROUNDS = true;
+    // the working value of the faces: the boundary as stored, or a deficit of 0
+    static __device__ __forceinline__ float face(float bval) {
+        return EN == OLC_ENC_DEFICIT ? 0.0f : Store16<ST>::to_f(Store16<ST>::from_f(bval));
+    }
+    // rounded to storage (voxel index vox) and back
+    static __device__ __forceinline__ float4 round(float4 v, olc_u32 vox, olc_u32 key) {
+        if (IsSR<ST>::value)
+            return value(make_uint2(pack2_sr<ST>(v.x, v.y, olc_sr_pair(vox >> 1, key)),
+                                    pack2_sr<ST>(v.z, v.w, olc_sr_pair((vox >> 1) + 1, key))));
+        return value(make_uint2(pack2<ST>(v.x, v.y), pack2<ST>(v.z, v.w)));
+    }
+    struct Update {
+        f32x2 r2, idl, idr, dsl, dsr;
+        float4 lo;
+        float b;
+        __device__ __forceinline__ Update(const ResidentArgs& a, float bval, const bool (&f)[4]) {
+            const float ds = EN == OLC_ENC_DEFICIT ? a.dec_sub : 0.0f;
+            r2 = pk2(a.r, a.r);
+            idl = pk2(f[0] ? 0.0f : a.inv_decay, f[1] ? 0.0f : a.inv_decay);
+            idr = pk2(f[2] ? 0.0f : a.inv_decay, f[3] ? 0.0f : a.inv_decay);
+            dsl = pk2(f[0] ? 0.0f : ds, f[1] ? 0.0f : ds);
+            dsr = pk2(f[2] ? 0.0f : ds, f[3] ? 0.0f : ds);
+            lo = make_float4(f[0] ? bval : 0.0f, f[1] ? bval : 0.0f, f[2] ? bval : 0.0f, f[3] ? bval : 0.0f);
+            b = a.bval;
+        }
+        __device__ __forceinline__ float4 operator()(float xl, float xr, const float4& c, const float4& ym,
+                                                     const float4& yp, const float4& zm, const float4& zp) const {
+            const float4 v = stencil_update4h<EN>(xl, xr, c, ym, yp, zm, zp, r2, idl, idr, dsl, dsr);
+            const float4 w = make_float4(fmaxf(v.x, lo.x), fmaxf(v.y, lo.y), fmaxf(v.z, lo.z), fmaxf(v.w, lo.w));
+            if (EN != OLC_ENC_DEFICIT) return w;
+            return make_float4(fminf(w.x, b), fminf(w.y, b), fminf(w.z, b), fminf(w.w, b));
+        }
+    };
 };
 
 __device__ __forceinline__ float4 lds4(olc_u32 p) {
@@ -128,7 +230,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const ResidentArgs a) {
     const int rows = min(a.By, a.ny - y0), planes = min(a.Bz, a.nz - z0);
     const olc_u32 sy = (olc_u32)a.nx, sz = (olc_u32)a.nx * (olc_u32)a.ny;
     const int tid = threadIdx.x, lane = tid & 31;
-    const float bval = a.bval;
+    const float bval = E::face(a.bval);  // what the faces hold
     const float4 b4 = make_float4(bval, bval, bval, bval);
 
     // this thread's column of the tile; threads without one work on some other
@@ -150,13 +252,8 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const ResidentArgs a) {
         work |= inner ? 1u << k : 0u;
         publish |= inner && (ry == 0 || ry == rows - 1 || kz0 + k == 0 || kz0 + k == planes - 1) ? 1u << k : 0u;
     }
-    // x faces (and what lies beyond a row's end): a factor 0 and a lower bound
-    // bval in the clamp that every voxel has
-    const bool f0 = x == 0 || left <= 1, f1 = left <= 2, f2 = left <= 3, f3 = left <= 4;
-    const f32x2 idl = pk2(f0 ? 0.0f : a.inv_decay, f1 ? 0.0f : a.inv_decay);
-    const f32x2 idr = pk2(f2 ? 0.0f : a.inv_decay, f3 ? 0.0f : a.inv_decay);
-    const float4 lo = make_float4(f0 ? bval : 0.0f, f1 ? bval : 0.0f, f2 ? bval : 0.0f, f3 ? bval : 0.0f);
-    const f32x2 r2 = pk2(a.r, a.r), nz2 = pk2(a.neg_zero, a.neg_zero);
+    const bool face[4] = {x == 0 || left <= 1, left <= 2, left <= 3, left <= 4};  // x faces, and beyond the row's end
+    const typename E::Update update(a, bval, face);
     // WRAP: rows go on in the next warp; its first and last lanes read their x
     // neighbours from shared memory
     const olc_u32 need_l = WRAP && lane == 0 && x > 0, need_r = WRAP && lane == 31 && left > 4;
@@ -251,6 +348,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const ResidentArgs a) {
     }
     __syncthreads();
 
+    const olc_u32 step = E::ROUNDS ? (a.step_ctr ? *a.step_ctr : a.step_host) : 0u;
     bool gave_up = false;
     olc_u32 spins = 0;
     for (int e = 0;; ++e) {
@@ -259,6 +357,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const ResidentArgs a) {
         void* out = (e & 1) ? a.in : a.other;
         const olc_u32 phase = (e & 2) ? 0u : E::PHASE;
         const olc_u32 publish_now = last ? 0u : publish;
+        const olc_u32 key = E::ROUNDS ? olc_sr_key(step, a.sub0 + e, a.field) : 0u;
         spins = 0;
         // ---- one substep of the own column
         if (busy) {
@@ -277,7 +376,8 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const ResidentArgs a) {
                     asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; @p ld.shared.f32 %0, [%1 + 16]; }"
                                  : "+f"(xr) : "r"(pc), "r"(need_r));
                 }
-                const float4 v = stencil_update4g(xl, xr, c[k], lds4(pm), lds4(pp), prev, lds4(pz), r2, idl, idr, lo, nz2);
+                float4 v = update(xl, xr, c[k], lds4(pm), lds4(pp), prev, lds4(pz));
+                if (E::ROUNDS) v = E::round(v, vo, key);
                 prev = c[k];
                 if (work >> k & 1u) {
                     c[k] = v;
@@ -423,7 +523,8 @@ cudaError_t launch_resident_t(const ResidentArgs& a, const ResidentPlan& p, cuda
 
 template <int K, int NT, class E>
 cudaError_t launch_resident_k(const ResidentArgs& a, const ResidentPlan& p, cudaStream_t s) {
-    if (!E::GROUPS) return launch_resident_t<K, NT, RING_ITEMS, true, E>(a, p, s);
+    // one variant serves rows read by words, and 16-bit storage
+    if (!E::GROUPS || E::ROUNDS) return launch_resident_t<K, NT, RING_ITEMS, true, E>(a, p, s);
     const bool wrap = a.G > 32 || (32 % a.G) != 0;
     if (p.RI == 1)
         return wrap ? launch_resident_t<K, NT, 1, true, E>(a, p, s) : launch_resident_t<K, NT, 1, false, E>(a, p, s);
@@ -450,6 +551,29 @@ bool resident_fits(const FieldStep& fs) {
     return make_resident_plan(fs.dims, (fs.dims[0] & 3) == 0, device_sms(), &p);
 }
 
+static void fill_resident_args(ResidentArgs* a, void* in, void* other, const FieldStep& fs, const ResidentPlan& p,
+                               int substeps, olc_u32* status) {
+    *a = ResidentArgs{};
+    a->in = in;
+    a->other = other;
+    a->nx = fs.dims[0];
+    a->ny = fs.dims[1];
+    a->nz = fs.dims[2];
+    a->G = (a->nx + 3) / 4;
+    a->By = p.By;
+    a->Bz = p.Bz;
+    a->ty = p.ty;
+    a->runs = p.runs;
+    a->L = p.L;
+    a->substeps = substeps;
+    a->r = fs.r;
+    a->inv_decay = fs.inv_decay;
+    a->bval = fs.bval;
+    a->neg_zero = -0.0f;
+    a->status = status;
+    a->dec_sub = fs.dec_sub;
+}
+
 // `substeps` substeps from `in` (both buffers hold substep results: clear sign
 // bits); returns the buffer holding the result, or null when the launch was
 // not possible.
@@ -459,24 +583,38 @@ float* run_resident(float* in, float* other, const FieldStep& fs, int substeps, 
     ResidentPlan p;
     if (substeps < 1 || !make_resident_plan(fs.dims, vec, device_sms(), &p)) return nullptr;
     ResidentArgs a;
-    a.in = in;
-    a.other = other;
-    a.nx = fs.dims[0];
-    a.ny = fs.dims[1];
-    a.nz = fs.dims[2];
-    a.G = (a.nx + 3) / 4;
-    a.By = p.By;
-    a.Bz = p.Bz;
-    a.ty = p.ty;
-    a.runs = p.runs;
-    a.L = p.L;
-    a.substeps = substeps;
-    a.r = fs.r;
-    a.inv_decay = fs.inv_decay;
-    a.bval = fs.bval;
-    a.neg_zero = -0.0f;
-    a.status = status;
+    fill_resident_args(&a, in, other, fs, p, substeps, status);
     const cudaError_t e = vec ? launch_resident<ResidentF32<true>>(a, p, s) : launch_resident<ResidentF32<false>>(a, p, s);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return (substeps & 1) ? other : in;
+}
+
+bool resident_fits16(const FieldStep& fs) {
+    return fs.encoding != OLC_ENC_OFFSET3 && resident_fits(fs);
+}
+
+// The same for 16-bit storage: substeps sub0 .. sub0 + substeps - 1.
+void* run_resident16(void* in, void* other, const FieldStep& fs, int substeps, olc_u32* status, const olc_u32* step_ctr,
+                     olc_u32 step_host, int sub0, int field, cudaStream_t s) {
+    ResidentPlan p;
+    if (substeps < 1 || fs.encoding == OLC_ENC_OFFSET3 || !make_resident_plan(fs.dims, true, device_sms(), &p))
+        return nullptr;
+    ResidentArgs a;
+    fill_resident_args(&a, in, other, fs, p, substeps, status);
+    a.step_ctr = step_ctr;
+    a.step_host = step_host;
+    a.sub0 = sub0;
+    a.field = field;
+    cudaError_t e = cudaErrorInvalidValue;
+    with_storage16(fs.storage, fs.encoding, [&](auto st, auto en) {
+        constexpr int ST = decltype(st)::value, EN = decltype(en)::value;
+        if constexpr (EN != OLC_ENC_OFFSET3) {
+            e = launch_resident<Resident16<ST, EN>>(a, p, s);
+        }
+    });
     if (e != cudaSuccess) {
         cudaGetLastError();
         return nullptr;

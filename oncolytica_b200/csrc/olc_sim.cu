@@ -376,7 +376,7 @@ int step_once(OlcSim* s, int collect, cudaStream_t st) {
                                        s->counters + OLC_CTR_STATUS, s->counters + OLC_CTR_FIELD_STEP, 0u, (int)f, st);
             s->field_cur[f] = (res == s->field[cur][f]) ? cur : 1 - cur;
             substeps += (uint32_t)s->fstep[f].substeps;
-            launches += (uint64_t)s->fstep[f].substeps;
+            launches += (uint64_t)(resident_fits16(s->fstep[f]) ? RESIDENT_LEAD + 1 : s->fstep[f].substeps);
             continue;
         }
         float* a = s->field[cur][f];

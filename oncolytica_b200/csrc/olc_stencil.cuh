@@ -109,14 +109,6 @@ __device__ __forceinline__ float4 stencil_update4f(float xl, float xr, const flo
     return make_float4(fmaxf(v.x, lo_l), fmaxf(v.y, 0.0f), fmaxf(v.z, 0.0f), fmaxf(v.w, lo_r));
 }
 
-// stencil_update4f with a lower bound for each voxel.
-__device__ __forceinline__ float4 stencil_update4g(float xl, float xr, const float4& c, const float4& ym,
-                                                   const float4& yp, const float4& zm, const float4& zp, f32x2 r2,
-                                                   f32x2 idl, f32x2 idr, const float4& lo, f32x2 nz2) {
-    const float4 v = stencil_update4u(xl, xr, c, ym, yp, zm, zp, r2, idl, idr, nz2);
-    return make_float4(fmaxf(v.x, lo.x), fmaxf(v.y, lo.y), fmaxf(v.z, lo.z), fmaxf(v.w, lo.w));
-}
-
 // The update of the 16-bit field storages: the same sums, with the two
 // products fused into their sums (one rounding each):
 //   u = fma(r, fma(-6, c, s), c),   out = max(u * inv_decay, 0)
@@ -140,6 +132,23 @@ __device__ __forceinline__ void stencil_update8_fma(float xl, float xr, const fl
         out[e] = fmaxf(w.x, 0.0f);
         out[e + 1] = fmaxf(w.y, 0.0f);
     }
+}
+
+// stencil_update8_fma on four voxels (not yet clamped), the decay factors and,
+// for OLC_ENC_DEFICIT, the decay terms given per pair.
+template <int EN>
+__device__ __forceinline__ float4 stencil_update4h(float xl, float xr, const float4& c, const float4& ym,
+                                                   const float4& yp, const float4& zm, const float4& zp, f32x2 r2,
+                                                   f32x2 idl, f32x2 idr, f32x2 dsl, f32x2 dsr) {
+    const f32x2 m6 = pk2(-6.0f, -6.0f);
+    const f32x2 c0 = pk2(c.x, c.y), c1 = pk2(c.z, c.w);
+    const f32x2 x0 = pk2(__fadd_rn(xl, c.y), __fadd_rn(c.x, c.z)), x1 = pk2(__fadd_rn(c.y, c.w), __fadd_rn(c.z, xr));
+    const f32x2 s0 = add2(add2(x0, add2(pk2(ym.x, ym.y), pk2(yp.x, yp.y))), add2(pk2(zm.x, zm.y), pk2(zp.x, zp.y)));
+    const f32x2 s1 = add2(add2(x1, add2(pk2(ym.z, ym.w), pk2(yp.z, yp.w))), add2(pk2(zm.z, zm.w), pk2(zp.z, zp.w)));
+    const f32x2 u0 = fma2(r2, fma2(m6, c0, s0), c0), u1 = fma2(r2, fma2(m6, c1, s1), c1);
+    const float2 a = upk2(EN == OLC_ENC_DEFICIT ? fma2(u0, idl, dsl) : mul2(u0, idl));
+    const float2 b = upk2(EN == OLC_ENC_DEFICIT ? fma2(u1, idr, dsr) : mul2(u1, idr));
+    return make_float4(a.x, a.y, b.x, b.y);
 }
 
 // stencil_update8_fma on the working values of an encoded 16-bit field

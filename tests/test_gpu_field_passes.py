@@ -77,3 +77,35 @@ def test_two_substeps_per_pass_leave_negative_boundaries_to_single_passes(cuda, 
 
 def test_large_field_takes_two_substeps_per_pass_by_itself(cuda, olc):
     _diffuse(cuda, olc, (256, 130, 140), 7, boundary=0.5)
+
+
+@pytest.mark.parametrize("storage,encoding", [(1, 0), (2, 0), (3, 0), (4, 0), (2, 1), (3, 1)])
+@pytest.mark.parametrize("dims,substeps", [((8, 3, 3), 6), ((24, 20, 19), 7), ((136, 17, 9), 6), ((64, 61, 67), 9)])
+def test_resident_16_bit_field_bit_exact(cuda, olc, dims, substeps, storage, encoding):
+    """The same on 16-bit storage holding values or deficits, rounded to nearest
+    and stochastically: two steps with uptake, residuals included."""
+    import torch
+
+    nx, ny, nz = dims
+    rng = np.random.default_rng(sum(dims) + storage)
+    f = (0.05 + 0.6 * rng.random((nz, ny, nx))).astype(np.float32)
+    bits = oracle.to_bits16(f, storage, encoding, 0.7)
+    comp = np.zeros_like(f)
+    fd = torch.from_numpy(bits.view(np.int16).copy()).to(cuda)
+    tmp = torch.from_numpy(rng.integers(-32768, 32767, f.shape).astype(np.int16)).to(cuda)
+    cd = torch.zeros(f.size, dtype=torch.float32, device=cuda)
+    dt = 0.15 * substeps
+    spec = _lib.OlcDiffusion(diffusion=1.0, decay=0.05, boundary=0.7, substeps=substeps, has_sink=1, storage=storage,
+                             encoding=encoding)
+    dims_c = (C.c_int32 * 3)(nx, ny, nz)
+    for step in range(2):
+        sink = np.where(rng.random(f.shape) < 0.2, 0.5 * rng.random(f.shape), 0.0).astype(np.float32)
+        sd = torch.from_numpy(sink.copy()).to(cuda)
+        bits, comp = oracle.diffuse16(bits, sink, comp, 1.0, dt, 1.0, 0.05, 0.7, substeps, storage, step=5 + step,
+                                      field=2, encoding=encoding)
+        _lib.check(olc.olc_stage_diffuse16(C.c_void_p(fd.data_ptr()), C.c_void_p(tmp.data_ptr()),
+                                           C.c_void_p(sd.data_ptr()), C.c_void_p(cd.data_ptr()), C.byref(dims_c), 1.0,
+                                           dt, C.byref(spec), 5 + step, 2, None))
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(fd.cpu().numpy().view(np.uint16).reshape(f.shape), bits)
+        np.testing.assert_array_equal(cd.cpu().numpy().reshape(f.shape), comp)
