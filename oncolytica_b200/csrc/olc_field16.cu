@@ -122,19 +122,30 @@ void launch_react16(void* f, float* sink, float* comp, const FieldStep& fs, cuda
 }
 
 // ------------------------------------------------------------------ diffusion substep
-// The TMA tile of k_substep_x4 on 16-bit storage, eight voxels per thread: a
-// CTA of 8 x TYR threads owns a 64 x TYR x TZ block; the TMA box is
-// 80 x (TYR+2) x (TZ+2) elements with x starting 8 columns early (16-byte
-// alignment of 2-byte elements).  Per eight voxels a thread issues 16-byte
-// shared loads of the centre, y and z rows, two 2-byte loads of the x
-// neighbours and one 16-byte store, as many instructions per byte as the
-// 4-wide FP32 kernel.
+// A CTA owns a 64 x TYR x TZ block; the TMA box is 80 x (TYR+2) x (TZ+2)
+// elements with x starting 8 columns early (16-byte alignment of 2-byte
+// elements).  The substep is bound by instruction issue: by the stencil in the
+// value and deficit encodings, where a thread walks one row of eight x voxels
+// up z (t16_tile8), and by decoding and encoding the elements in the
+// three-offset one.  There a thread owns four x voxels of four rows and keeps
+// two planes of them decoded in registers (t16_tile4): an element is decoded
+// 1.5 times (its own row's plane once, the groups' outer rows once more), by
+// the other walk 3.25 times.  The x neighbours come from the neighbour lanes;
+// the columns next to the block are decoded once per plane, one value per lane.
+// BF16-SR, 256^3, us per three-offset substep: 43.8 with the rows of eight and
+// an element at a time coded by compares; 30.8 with pairs coded by integer
+// arithmetic (Codec::work2, pack3); 29.2 with the four-row walk too; 27.0 with
+// tiles of 4 planes.  In the value encoding decoding is one instruction.
 namespace t16 {
 constexpr int TX = 64, HX = 8, WX = TX + 2 * HX;  // 80 elements, 160 bytes
-constexpr int TYR = 16, TZ = 8, WY = TYR + 2, WZ = TZ + 2;
-constexpr int THREADS = 8 * TYR;
-constexpr unsigned BYTES = WX * WY * WZ * 2;
-constexpr size_t SMEM = BYTES + 16 + 128;
+constexpr int TYR = 16, TZ = 8, WY = TYR + 2;  // TZ: planes per tile, but for the four-row walk outside batches
+constexpr int R = 4;  // rows per thread of the four-row walk
+__host__ __device__ constexpr bool four_rows(int en) { return en == OLC_ENC_OFFSET3; }
+__host__ __device__ constexpr int threads(int en) { return four_rows(en) ? TX / 4 * (TYR / R) : TX / 8 * TYR; }
+__host__ __device__ constexpr unsigned bytes(int tz) { return WX * WY * (tz + 2) * 2; }
+constexpr unsigned BYTES = bytes(TZ);
+constexpr size_t smem(int tz) { return bytes(tz) + 16 + 128; }
+constexpr size_t SMEM = smem(TZ);
 }  // namespace t16
 
 // The working value the Dirichlet faces hold (OLC_ENC_*): the boundary as
@@ -149,7 +160,7 @@ __device__ __forceinline__ float face_work(float bval) {
 // The 64 x TYR x TZ output block at (x0, y0, z0) from its staged 16-bit box
 // (stochastic-rounding key given), on the working values of encoding EN.
 template <int ST, int EN>
-__device__ __forceinline__ void t16_tile(const unsigned short* tile, unsigned short* __restrict__ out, int x0, int y0,
+__device__ __forceinline__ void t16_tile8(const unsigned short* tile, unsigned short* __restrict__ out, int x0, int y0,
                                          int z0, int nx, int ny, int nz, const FieldStep& fs, olc_u32 key) {
     using namespace t16;
     const int g = threadIdx.x & 7, ty = threadIdx.x >> 3;
@@ -200,20 +211,101 @@ __device__ __forceinline__ void t16_tile(const unsigned short* tile, unsigned sh
     }
 }
 
+// The same for the 64 x TYR x tz block, with four rows of four voxels per thread.
 template <int ST, int EN>
-__global__ void __launch_bounds__(t16::THREADS) k_substep16(const __grid_constant__ CUtensorMap in_map,
+__device__ __forceinline__ void t16_tile4(const unsigned short* tile, unsigned short* __restrict__ out, int x0, int y0,
+                                         int z0, int nx, int ny, int nz, int tz, const FieldStep& fs, olc_u32 key) {
+    using namespace t16;
+    const int lx = threadIdx.x & 15, gr = threadIdx.x >> 4, lane = threadIdx.x & 31;
+    const int x = x0 + 4 * lx, y = y0 + R * gr;
+    const EncConst k = enc_const(fs);
+    constexpr int PS = WY * WX;
+    const unsigned short* col = tile + (R * gr + 1) * WX + HX + 4 * lx;  // plane 0 of this thread's first row
+    // the columns next to the block: lanes 0..3 of each 16 hold the left one's
+    // rows, lanes 8..11 the right one's
+    const unsigned short* edge = tile + (R * gr + 1 + (lx & 3)) * WX + ((lx & 8) ? HX + TX : HX - 1);
+    const int edge_src = (lane & 16) + (lx == 0 ? 0 : 8);
+    const bool first = lx == 0, final = lx == 15, ex0 = x == 0, ex3 = x + 3 == nx - 1;
+    const float bf = face_work<ST, EN>(fs.bval);
+    const float4 b4 = make_float4(bf, bf, bf, bf);
+    const f32x2 r2 = pk2(fs.r, fs.r), id2 = pk2(fs.inv_decay, fs.inv_decay), ds2 = pk2(fs.dec_sub, fs.dec_sub);
+    const olc_u32 sz = (olc_u32)nx * (olc_u32)ny;
+    olc_u32 vi = (olc_u32)z0 * sz + (olc_u32)y * (olc_u32)nx + (olc_u32)x;  // low 32 bits are all the hash takes
+    unsigned short* o = out + ((size_t)z0 * ny + y) * nx + x;
+    const int last = min(tz, nz - z0);
+    // lanes past the grid compute (inside the box), but store nothing
+    const int rows = x < nx ? min(R, ny - y) : 0;
+    const bool y_edge = y == 0 || y + R >= ny;
+    float4 A[R], B[R];  // planes z - 1 and z of the own rows, by turns
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+        A[m] = load4w<ST, EN>(col + m * WX, k);
+        B[m] = load4w<ST, EN>(col + PS + m * WX, k);
+    }
+    // output plane lz - 1 of the block; plane lz + 1 of the box replaces zm
+    auto plane = [&](int lz, float4 (&zm)[R], const float4 (&c)[R]) {
+        const int z = z0 + lz - 1;
+        const unsigned short* pc = col + lz * PS;
+        float4 ym = load4w<ST, EN>(pc - WX, k);
+        const float4 dn = load4w<ST, EN>(pc + R * WX, k);
+        const float ec = Codec<ST, EN>::work(edge[lz * PS], k);
+        const bool faces = y_edge || z == 0 || z == nz - 1;
+#pragma unroll
+        for (int m = 0; m < R; ++m) {
+            const float4 zp = load4w<ST, EN>(pc + PS + m * WX, k);
+            const float e = __shfl_sync(0xffffffffu, ec, edge_src + m);
+            float xl = __shfl_up_sync(0xffffffffu, c[m].w, 1, 16);
+            float xr = __shfl_down_sync(0xffffffffu, c[m].x, 1, 16);
+            xl = first ? e : xl;
+            xr = final ? e : xr;
+            float4 v = stencil_update4h<EN>(xl, xr, c[m], ym, m == R - 1 ? dn : c[m < R - 1 ? m + 1 : 0], zm[m], zp, r2,
+                                            id2, id2, ds2, ds2);
+            v = make_float4(fmaxf(v.x, 0.0f), fmaxf(v.y, 0.0f), fmaxf(v.z, 0.0f), fmaxf(v.w, 0.0f));
+            ym = c[m];
+            zm[m] = zp;
+            if (ex0) v.x = bf;
+            if (ex3) v.w = bf;
+            if (faces) {
+                const int yy = y + m;
+                if (yy == 0 || yy == ny - 1 || z == 0 || z == nz - 1) v = b4;
+            }
+            if (m < rows) store4w_at<ST, EN>(o + (size_t)m * nx, v, vi + (olc_u32)m * (olc_u32)nx, key, k);
+        }
+        o += (size_t)nx * ny;
+        vi += sz;
+    };
+#pragma unroll 1
+    for (int lz = 1; lz <= last; lz += 2) {
+        plane(lz, A, B);
+        if (lz < last) plane(lz + 1, B, A);
+    }
+}
+
+template <int ST, int EN>
+__device__ __forceinline__ void t16_tile(const unsigned short* tile, unsigned short* __restrict__ out, int x0, int y0,
+                                         int z0, int nx, int ny, int nz, int tz, const FieldStep& fs,
+                                         olc_u32 key) {
+    if (t16::four_rows(EN))
+        t16_tile4<ST, EN>(tile, out, x0, y0, z0, nx, ny, nz, tz, fs, key);
+    else
+        t16_tile8<ST, EN>(tile, out, x0, y0, z0, nx, ny, nz, fs, key);  // tz is TZ
+}
+
+template <int ST, int EN>
+__global__ void __launch_bounds__(t16::threads(EN)) k_substep16(const __grid_constant__ CUtensorMap in_map,
                                                            unsigned short* __restrict__ out, const FieldStep fs,
                                                            olc_u32* status, int rev, const olc_u32* step_ctr,
-                                                           olc_u32 step_host, int sub, int field) {
+                                                           olc_u32 step_host, int sub, int field, int tz_run) {
     using namespace t16;
+    const int tz = four_rows(EN) ? tz_run : TZ;
     extern __shared__ unsigned char t16_raw[];
     const olc_u32 pad = (128u - (smem_addr(t16_raw) & 127u)) & 127u;
     unsigned short* tile = reinterpret_cast<unsigned short*>(t16_raw + pad);
-    const olc_u32 bar = smem_addr(t16_raw + pad + BYTES);
+    const olc_u32 bar = smem_addr(t16_raw + pad + bytes(tz));
     const int bx = rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
     const int by = rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
     const int bz = rev ? gridDim.z - 1 - blockIdx.z : blockIdx.z;
-    const int x0 = bx * TX, y0 = by * TYR, z0 = bz * TZ;
+    const int x0 = bx * TX, y0 = by * TYR, z0 = bz * tz;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
@@ -223,7 +315,7 @@ __global__ void __launch_bounds__(t16::THREADS) k_substep16(const __grid_constan
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(BYTES) : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes(tz)) : "memory");
         asm volatile(
             "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
             "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_addr(tile)),
@@ -234,7 +326,7 @@ __global__ void __launch_bounds__(t16::THREADS) k_substep16(const __grid_constan
     // a warp leaves as a whole (the tile has no block-wide barrier)
     const bool tile_ready = olc_mbar_wait_bounded(bar, 0, status);
     if (__any_sync(0xffffffffu, !tile_ready)) return;
-    t16_tile<ST, EN>(tile, out, x0, y0, z0, fs.dims[0], fs.dims[1], fs.dims[2], fs,
+    t16_tile<ST, EN>(tile, out, x0, y0, z0, fs.dims[0], fs.dims[1], fs.dims[2], tz, fs,
                      olc_sr_key(step_ctr ? *step_ctr : step_host, sub, field));
 }
 
@@ -246,7 +338,7 @@ __global__ void __launch_bounds__(t16::THREADS) k_substep16(const __grid_constan
 static_assert(t16::TX == BATCH_T16_TX && t16::TYR == BATCH_T16_TY && t16::TZ == BATCH_T16_TZ, "batched 16-bit tile");
 
 template <int ST, int EN>
-__global__ void __launch_bounds__(t16::THREADS) k_substep_batch_t16(
+__global__ void __launch_bounds__(t16::threads(EN)) k_substep_batch_t16(
     const uint4* __restrict__ tiles, const OlcSimDesc* __restrict__ sims, const FieldStep* __restrict__ steps,
     const CUtensorMap* __restrict__ maps, int field, int n_fields, const unsigned char* __restrict__ fpar, int sub,
     unsigned short* fa, unsigned short* fb, const olc_u32* step_ctr, olc_u32* status) {
@@ -288,7 +380,7 @@ __global__ void __launch_bounds__(t16::THREADS) k_substep_batch_t16(
     // a warp leaves as a whole (the tile has no block-wide barrier)
     const bool tile_ready = olc_mbar_wait_bounded(bar, 0, status);
     if (__any_sync(0xffffffffu, !tile_ready)) return;
-    t16_tile<ST, EN>(tile, out, x0, y0, z0, d.cdims[0], d.cdims[1], d.cdims[2], fs,
+    t16_tile<ST, EN>(tile, out, x0, y0, z0, d.cdims[0], d.cdims[1], d.cdims[2], TZ, fs,
                      olc_sr_key(*step_ctr - d.step_base, sub, field));
 }
 
@@ -306,7 +398,7 @@ static void launch_bt16(const uint4* tiles, olc_u32 n_tiles, const OlcSimDesc* s
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_tiles);
-    cfg.blockDim = dim3(THREADS);
+    cfg.blockDim = dim3(threads(EN));
     cfg.dynamicSmemBytes = SMEM;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -329,17 +421,32 @@ void launch_substep_batch_t16(const BatchArgs& b, int storage, int encoding, con
     });
 }
 
-bool make_field_maps16(FieldMaps16* m, void* a, void* b, const int dims[3]) {
+bool make_field_maps16(FieldMaps16* m, void* a, void* b, const int dims[3], int encoding) {
     using namespace t16;
     m->ok = false;
-    const cuuint32_t box[3] = {WX, WY, WZ};
+    // The four-row walk's tiles are 4 planes deep, and shallower where these
+    // would be fewer than 12 per SM (a tile's planes follow one another, so few
+    // deep tiles leave the SMs waiting).  us per BF16-SR substep with 8, 4, 2
+    // and 1 planes: 256^3 27.8, 27.0, -, -; 200^3 20.8, 18.4, 19.4, -;
+    // 160^3 16.2, 11.4, 10.8, 11.9; 256 x 256 x 64 -, 11.2, 9.3, 10.3;
+    // 128^3 -, -, 7.0, 6.3; 32^3 -, -, 3.3, 2.6.
+    m->tz = TZ;
+    if (four_rows(encoding)) {
+        int sms = 148, dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const long long columns = (long long)((dims[0] + TX - 1) / TX) * ((dims[1] + TYR - 1) / TYR);
+        m->tz = 4;
+        while (m->tz > 1 && columns * ((dims[2] + m->tz - 1) / m->tz) < 12LL * sms) m->tz /= 2;
+    }
+    const cuuint32_t box[3] = {WX, WY, (cuuint32_t)(m->tz + 2)};
     if (!encode_map_elems(&m->map[0], a, dims, box, 2) || !encode_map_elems(&m->map[1], b, dims, box, 2)) return false;
     m->ok = true;
     return true;
 }
 
 template <int ST, int EN>
-static void launch_sub16(const CUtensorMap& map, void* out, const FieldStep& fs, olc_u32* status, int rev,
+static void launch_sub16(const CUtensorMap& map, int tz, void* out, const FieldStep& fs, olc_u32* status, int rev,
                          const olc_u32* step_ctr, olc_u32 step_host, int sub, int field, cudaStream_t s) {
     using namespace t16;
     static int configured_mask = 0;
@@ -350,9 +457,9 @@ static void launch_sub16(const CUtensorMap& map, void* out, const FieldStep& fs,
         configured_mask |= 1 << dev;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((fs.dims[0] + TX - 1) / TX, (fs.dims[1] + TYR - 1) / TYR, (fs.dims[2] + TZ - 1) / TZ);
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = SMEM;
+    cfg.gridDim = dim3((fs.dims[0] + TX - 1) / TX, (fs.dims[1] + TYR - 1) / TYR, (fs.dims[2] + tz - 1) / tz);
+    cfg.blockDim = dim3(threads(EN));
+    cfg.dynamicSmemBytes = smem(tz);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -360,7 +467,7 @@ static void launch_sub16(const CUtensorMap& map, void* out, const FieldStep& fs,
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, k_substep16<ST, EN>, map, static_cast<unsigned short*>(out), fs, status, rev, step_ctr,
-                       step_host, sub, field);
+                       step_host, sub, field, tz);
 }
 
 void* run_substeps16(void* a, void* b, const FieldMaps16& m, int a_index, const FieldStep& fs, olc_u32* status,
@@ -376,7 +483,7 @@ void* run_substeps16(void* a, void* b, const FieldMaps16& m, int a_index, const 
                                            field, s))
                 return res;
         with_storage16(fs.storage, fs.encoding, [&](auto st, auto en) {
-            launch_sub16<decltype(st)::value, decltype(en)::value>(m.map[cur], bufs[1 - cur], fs, status, i & 1,
+            launch_sub16<decltype(st)::value, decltype(en)::value>(m.map[cur], m.tz, bufs[1 - cur], fs, status, i & 1,
                                                                    step_ctr, step_host, i, field, s);
         });
         cur = 1 - cur;

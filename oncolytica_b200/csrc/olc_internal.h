@@ -183,9 +183,10 @@ bool encode_map_elems(CUtensorMap* map, void* base, const int dims[3], const cuu
 // substeps that round each result to the storage type.
 struct FieldMaps16 {
     bool ok = false;
+    int tz = 8;  // planes per tile of the substep
     CUtensorMap map[2];
 };
-bool make_field_maps16(FieldMaps16* m, void* a, void* b, const int dims[3]);
+bool make_field_maps16(FieldMaps16* m, void* a, void* b, const int dims[3], int encoding);
 void launch_react16(void* f, float* sink, float* comp, const FieldStep& fs, cudaStream_t s);
 // Runs fs.substeps substeps from buffer a_index of (a, b); returns the buffer holding the result.
 // step_ctr (device, else step_host) and field salt stochastic rounding.

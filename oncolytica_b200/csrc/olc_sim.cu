@@ -1285,7 +1285,7 @@ int olc_bind_field_ex(OlcSim* s, int index, void* a_, void* b_, float* sink, flo
         make_field_maps(&s->fmaps[index], a, b, s->geom.chem_dims, spec->boundary, s->tuning.stencil_tile_y,
                         s->tuning.stencil_tile_z,
                         s->tuning.stencil_pair_threads, s->tuning.stencil_pair_planes, s->tuning.stencil_l2_keep_pct);
-    if (spec->substeps > 0 && half && !make_field_maps16(&s->fmaps16[index], a, b, s->geom.chem_dims))
+    if (spec->substeps > 0 && half && !make_field_maps16(&s->fmaps16[index], a, b, s->geom.chem_dims, spec->encoding))
         return fail(s, OLC_ERR_ARG, "olc_bind_field_ex: TMA descriptors of the 16-bit field failed (16-byte aligned "
                                     "buffers, x extent a multiple of 8)");
     s->comp[index] = half ? comp : nullptr;
@@ -2546,7 +2546,7 @@ int olc_stage_diffuse16(void* f, void* tmp, float* sink, float* comp, const int3
     cudaStream_t st = as_stream(stream);
     olc_u32* status = stage_status_word();
     FieldMaps16 maps;
-    if (!status || !make_field_maps16(&maps, f, tmp, dims))
+    if (!status || !make_field_maps16(&maps, f, tmp, dims, spec->encoding))
         return fail(nullptr, OLC_ERR_ARG, "olc_stage_diffuse16: TMA descriptors failed (16-byte aligned buffers)");
     launch_react16(f, spec->has_sink ? sink : nullptr, comp, fs, st);
     void* res = run_substeps16(f, tmp, maps, 0, fs, status, nullptr, step, field, st);

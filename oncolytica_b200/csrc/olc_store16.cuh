@@ -5,6 +5,7 @@
 #include <type_traits>
 
 #include "olc_device.cuh"
+#include "olc_stencil.cuh"
 #include "../../include/olc.h"
 
 namespace olc {
@@ -68,19 +69,6 @@ __device__ __forceinline__ olc_u32 olc_sr_pair(unsigned long long pair, olc_u32 
     return x ^ (x >> 15);
 }
 
-// Eight consecutive values (16 bytes): load to FP32, store with rounding at
-// voxel index vi (a multiple of 8; stochastic for the _SR types).
-template <int ST>
-__device__ __forceinline__ void load8(const unsigned short* p, float (&f)[8]) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(p);
-    const olc_u32 w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        f[2 * k] = Store16<ST>::to_f((unsigned short)(w[k] & 0xffffu));
-        f[2 * k + 1] = Store16<ST>::to_f((unsigned short)(w[k] >> 16));
-    }
-}
-
 // Two FP32 values -> one word of two 16-bit values (a in the low half, b in
 // the high half).  cvt.*x2 converts its first source into the high half.
 template <int ST>
@@ -105,18 +93,6 @@ __device__ __forceinline__ olc_u32 pack2_sr(float a, float b, olc_u32 rnd) {
     else
         asm("cvt.rs.f16x2.f32 %0, %1, %2, %3;" : "=r"(d) : "f"(b), "f"(a), "r"(rnd));
     return d;
-}
-
-// Eight values (16 bytes) stored at voxel index vi (a multiple of 8), rounded
-// to nearest even or, for the _SR types, stochastically with the pair hash.
-template <int ST>
-__device__ __forceinline__ void store8_at(unsigned short* p, const float (&v)[8], unsigned long long vi, olc_u32 key) {
-    olc_u32 w[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        w[k] = IsSR<ST>::value ? pack2_sr<ST>(v[2 * k], v[2 * k + 1], olc_sr_pair((vi >> 1) + k, key))
-                               : pack2<ST>(v[2 * k], v[2 * k + 1]);
-    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 // ------------------------------------------------------------------ encodings
@@ -167,12 +143,50 @@ struct Codec {
         *code = d < 0.0f ? 0x8000u : 0x4000u;
         return fabsf(d);
     }
-    // two working values -> one word (a low, b high), nearest or stochastic
+    // OLC_ENC_OFFSET3, two working values >= 0 (no NaN) at once.  The integer and
+    // select work of split3 saturated the ALU pipe (77 % busy, the FP32 pipe 23 %),
+    // so the offsets are found with multiply-adds: the signs of f - b/4 and
+    // f - (b - b/4) (exact differences, so the signs are exact) saturate to 0 or 1,
+    // their sum n counts the offset in units of b/2, and f - n b/2 is split3's
+    // difference.  n then becomes code bits 14 (n = 1) and 15 (n = 2).
+    static __device__ __forceinline__ olc_u32 pack3(float f0, float f1, const EncConst& k, bool sr, olc_u32 rnd) {
+        const float huge = __uint_as_float(0x7f000000u);  // 2^127: twice, any nonzero difference exceeds 1
+        const f32x2 f = pk2(fminf(f0, k.b), fminf(f1, k.b)), huge2 = pk2(huge, huge);
+        const float2 lo = upk2(mul2(sub2(f, pk2(k.quarter_b, k.quarter_b)), huge2));
+        const float2 hi = upk2(mul2(sub2(f, pk2(k.upper_q, k.upper_q)), huge2));
+        const f32x2 n = add2(pk2(__saturatef(__fmaf_rn(lo.x, huge, 1.0f)), __saturatef(__fmaf_rn(lo.y, huge, 1.0f))),
+                             pk2(__saturatef(__fmul_rn(hi.x, huge)), __saturatef(__fmul_rn(hi.y, huge))));
+        const float2 d = upk2(fma2(n, pk2(-k.half_b, -k.half_b), f)), nn = upk2(n);
+        const olc_u32 w = sr ? pack2_sr<ST>(d.x, d.y, rnd) : pack2<ST>(d.x, d.y);
+        // n0 and n1 in the halves' bits 0..1, from the mantissa of 2^23 + n0 + 2^16 n1
+        const olc_u32 m = __float_as_uint(__fadd_rn(__fmaf_rn(nn.y, 65536.0f, nn.x), 8388608.0f));
+        const olc_u32 c14 = m * 0x4000u, c13 = m * 0x2000u;  // bit 14: n = 1, bit 15: n = 2; the same one bit lower
+        // bit 15: the distance is negative or n = 2; bit 14: n = 2, or n = 1 and it is not negative
+        const olc_u32 t = (c14 & ~(w >> 1)) | c13;
+        return w | ((c14 & 0x80008000u) | (t & 0x40004000u));
+    }
+    // two working values, >= 0 and no NaN -> one word (a low, b high), nearest
+    // or stochastic (a magnitude rounds alike under either sign)
     static __device__ __forceinline__ olc_u32 pack(float a, float b, const EncConst& k, bool sr, olc_u32 rnd) {
         if (EN != OLC_ENC_OFFSET3) return sr ? pack2_sr<ST>(a, b, rnd) : pack2<ST>(a, b);
-        olc_u32 ca, cb;
-        const float ma = split3(a, k, &ca), mb = split3(b, k, &cb);
-        return (sr ? pack2_sr<ST>(ma, mb, rnd) : pack2<ST>(ma, mb)) | ca | (cb << 16);
+        return pack3(a, b, k, sr, rnd);
+    }
+    // the working values of a word's two elements
+    static __device__ __forceinline__ float2 work2(olc_u32 w, const EncConst& k) {
+        if (EN != OLC_ENC_OFFSET3)
+            return make_float2(Store16<ST>::to_f((unsigned short)(w & 0xffffu)), Store16<ST>::to_f((unsigned short)(w >> 16)));
+        // the offset's count n = floor(2 u + 1/2), u the element's 16 bits as a
+        // fraction: the high word of a 64-bit multiply-add, which adds the bits of
+        // 2^23 too, so that it reads as the float 2^23 + n (the compiler makes
+        // shifts and carries of it; kept a multiply by a hidden 2, a substep of
+        // 256^3 took 31.1 us instead of 29.2)
+        const olc_u64 half = ((olc_u64)0x4B000000u << 32) | 0x80000000u;
+        const olc_u32 n0 = (olc_u32)(((olc_u64)(w << 16) * 2u + half) >> 32);
+        const olc_u32 n1 = (olc_u32)(((olc_u64)w * 2u + half) >> 32);
+        const olc_u32 m = w & 0xBFFFBFFFu;
+        const f32x2 n = add2(pk2(__uint_as_float(n0), __uint_as_float(n1)), pk2(-8388608.0f, -8388608.0f));
+        return upk2(fma2(n, pk2(k.half_b, k.half_b),
+                         pk2(Store16<ST>::to_f((unsigned short)(m & 0xffffu)), Store16<ST>::to_f((unsigned short)(m >> 16)))));
     }
     // one working value -> one element, to nearest
     static __device__ __forceinline__ unsigned short enc_rn(float w, const EncConst& k) {
@@ -186,16 +200,13 @@ struct Codec {
 // Eight elements (16 bytes) to working values.
 template <int ST, int EN>
 __device__ __forceinline__ void load8w(const unsigned short* p, float (&f)[8], const EncConst& k) {
-    if (EN != OLC_ENC_OFFSET3) {
-        load8<ST>(p, f);
-        return;
-    }
     const uint4 raw = *reinterpret_cast<const uint4*>(p);
     const olc_u32 w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        f[2 * q] = Codec<ST, EN>::work((unsigned short)(w[q] & 0xffffu), k);
-        f[2 * q + 1] = Codec<ST, EN>::work((unsigned short)(w[q] >> 16), k);
+        const float2 v = Codec<ST, EN>::work2(w[q], k);
+        f[2 * q] = v.x;
+        f[2 * q + 1] = v.y;
     }
 }
 
@@ -209,6 +220,24 @@ __device__ __forceinline__ void store8w_at(unsigned short* p, const float (&v)[8
         w[q] = Codec<ST, EN>::pack(v[2 * q], v[2 * q + 1], k, IsSR<ST>::value,
                                    IsSR<ST>::value ? olc_sr_pair((vi >> 1) + q, key) : 0u);
     *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Four elements (8 bytes) to working values.
+template <int ST, int EN>
+__device__ __forceinline__ float4 load4w(const unsigned short* p, const EncConst& k) {
+    const uint2 w = *reinterpret_cast<const uint2*>(p);
+    const float2 a = Codec<ST, EN>::work2(w.x, k), b = Codec<ST, EN>::work2(w.y, k);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// Four working values stored at voxel index vi (a multiple of 4).
+template <int ST, int EN>
+__device__ __forceinline__ void store4w_at(unsigned short* p, const float4& v, olc_u32 vi, olc_u32 key,
+                                           const EncConst& k) {
+    const olc_u32 r0 = IsSR<ST>::value ? olc_sr_pair(vi >> 1, key) : 0u;
+    const olc_u32 r1 = IsSR<ST>::value ? olc_sr_pair((vi >> 1) + 1, key) : 0u;
+    *reinterpret_cast<uint2*>(p) = make_uint2(Codec<ST, EN>::pack(v.x, v.y, k, IsSR<ST>::value, r0),
+                                              Codec<ST, EN>::pack(v.z, v.w, k, IsSR<ST>::value, r1));
 }
 
 // The per-step reaction of one interior voxel (FS: a FieldStep): working value

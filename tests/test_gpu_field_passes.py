@@ -109,3 +109,33 @@ def test_resident_16_bit_field_bit_exact(cuda, olc, dims, substeps, storage, enc
         torch.cuda.synchronize()
         np.testing.assert_array_equal(fd.cpu().numpy().view(np.uint16).reshape(f.shape), bits)
         np.testing.assert_array_equal(cd.cpu().numpy().reshape(f.shape), comp)
+
+
+@pytest.mark.parametrize("storage", [1, 2, 3, 4])
+@pytest.mark.parametrize("dims", [(8, 3, 3), (72, 41, 37), (8, 2361, 23), (8, 2353, 47), (136, 17, 9)])
+def test_three_offset_substeps_bit_exact(cuda, olc, dims, storage):
+    """Tiles of one, two and four planes of the three-offset encoding, over
+    values at and on either side of its offsets' limits."""
+    import torch
+
+    nx, ny, nz = dims
+    b = np.float32(0.7)
+    rng = np.random.default_rng(sum(dims) + storage)
+    f = (1.2 * b * rng.random((nz, ny, nx))).astype(np.float32)
+    at = rng.random(f.shape) < 0.3
+    f[at] = rng.choice(np.array([0, b / 4, b / 2, b - b / 4, b], np.float32), int(at.sum()))
+    bits = oracle.to_bits16(f, storage, 2, b)
+    fd = torch.from_numpy(bits.view(np.int16).copy()).to(cuda)
+    tmp = torch.from_numpy(rng.integers(-32768, 32767, f.shape).astype(np.int16)).to(cuda)
+    cd = torch.zeros(f.size, dtype=torch.float32, device=cuda)
+    spec = _lib.OlcDiffusion(diffusion=1.0, decay=0.05, boundary=float(b), substeps=3, has_sink=0, storage=storage,
+                             encoding=2)
+    bits, comp = oracle.diffuse16(bits, None, np.zeros_like(f), 1.0, 0.45, 1.0, 0.05, float(b), 3, storage, step=9,
+                                  field=1, encoding=2)
+    dims_c = (C.c_int32 * 3)(nx, ny, nz)
+    _lib.check(olc.olc_stage_diffuse16(C.c_void_p(fd.data_ptr()), C.c_void_p(tmp.data_ptr()), None,
+                                       C.c_void_p(cd.data_ptr()), C.byref(dims_c), 1.0, 0.45, C.byref(spec), 9, 1,
+                                       None))
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(fd.cpu().numpy().view(np.uint16).reshape(f.shape), bits)
+    np.testing.assert_array_equal(cd.cpu().numpy().reshape(f.shape), comp)
