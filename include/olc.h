@@ -148,7 +148,7 @@ typedef struct {
  * gives the same bits; oncolytica_b200.autotune measures them on the
  * caller's workload and sets the fastest.  No counterpart in the reference
  * (its dispatches are fixed 256-wide: _gpu_backend.py:134-136). */
-#define OLC_CONTACT_FLAT   0  /* one flat walk over each agent's listed non-empty Moore bins */
+#define OLC_CONTACT_FLAT   0  /* lists each agent's near candidates, then computes their forces */
 #define OLC_CONTACT_NESTED 1  /* nested loops over the 27 Moore bins                       */
 typedef struct {
     int32_t stencil_tile_y;   /* tile of an FP32 one-substep pass: rows (8 or 16) ...  */

@@ -13,7 +13,7 @@
 // then y, then z; within a bin by sorted row.  The force sum follows that
 // order with separately rounded operations.
 #include "olc_internal.h"
-
+#include "olc_contact.cuh"
 
 namespace olc {
 
@@ -266,132 +266,66 @@ void launch_contact_mech(const float4* posr, const olc_u32* ranges, const olc_u3
                                           z);
 }
 
-// The same sum as k_contact with one flat loop over each agent's candidates:
-// a thread first lists its non-empty Moore bins (in order) in its own column
-// of shared memory, then walks rows bin after bin, so the lanes of a warp stay
-// converged until each has run out of candidates (the nested loops run every
-// bin as long as the fullest lane's), and it requests the next candidate's
-// record before using the current one (the pass waits on L2 latency).  Same
-// candidates, order and arithmetic.
-// One candidate of the flat walk: the pair law of k_contact, summed into f.
-__device__ __forceinline__ void contact_pair(const float4& p, const float4& q, olc_u32 i, olc_u32 j,
-                                             const ContactDev& c, float& fx, float& fy, float& fz) {
-    if (j == i || q.w < 0.0f) return;
-    const float ddx = __fsub_rn(p.x, q.x);
-    const float ddy = __fsub_rn(p.y, q.y);
-    const float ddz = __fsub_rn(p.z, q.z);
-    const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(ddx, ddx), __fmul_rn(ddy, ddy)), __fmul_rn(ddz, ddz));
-    const float rsum = __fadd_rn(p.w, q.w);
-    if (d2 > __fmul_rn(__fmul_rn(rsum, rsum), 1.00000095367431640625f)) return;
-    const float dist = sqrtf(d2);
-    if (!(dist < rsum)) return;
-    const float ov = __fsub_rn(rsum, dist);
-    const float f = __fmul_rn(__fmul_rn(c.stiffness, ov), sqrtf(ov));
-    if (dist < 1e-5f) {
-        fx = __fadd_rn(fx, i < j ? -f : f);
-    } else {
-        const float sc = __fdiv_rn(f, dist);
-        fx = __fadd_rn(fx, __fmul_rn(ddx, sc));
-        fy = __fadd_rn(fy, __fmul_rn(ddy, sc));
-        fz = __fadd_rn(fz, __fmul_rn(ddz, sc));
-    }
-}
-
-constexpr int CF_THREADS = 128;
+// The same sum as k_contact by contact_force_thread.
+constexpr int CF_THREADS = 64, CF_HITS = 24;
 __global__ void __launch_bounds__(CF_THREADS) k_contact_flat(const float4* __restrict__ posr,
                                                             const uint2* __restrict__ ranges, const olc_u32* n_dev,
-                                                            olc_u32 n_host, ContactDev c, float* __restrict__ xo,
-                                                            float* __restrict__ yo, float* __restrict__ zo) {
-    __shared__ uint2 s_bins[27][CF_THREADS];
+                                                            olc_u32 n_host, const __grid_constant__ ContactDev c,
+                                                            float* __restrict__ xo, float* __restrict__ yo,
+                                                            float* __restrict__ zo) {
+    __shared__ uint2 s_runs[CONTACT_RUNS][CF_THREADS];
+    __shared__ olc_u32 s_hits[CF_HITS][CF_THREADS];
     const olc_u32 n = n_dev ? *n_dev : n_host;
-    const float md = __fmul_rn(c.mobility, c.dt);
-    const int t = threadIdx.x;
-    for (olc_u32 base = blockIdx.x * CF_THREADS; base < n; base += gridDim.x * CF_THREADS) {
-        const olc_u32 i = base + t;
-        if (i >= n) continue;
-        const float4 p = posr[i];
-        if (p.w < 0.0f) continue;  // dead this step: no move, no force
-        const int cx = olc_bin_coord(p.x, c.tvs, c.tdims[0]);
-        const int cy = olc_bin_coord(p.y, c.tvs, c.tdims[1]);
-        const int cz = olc_bin_coord(p.z, c.tvs, c.tdims[2]);
-        // per-axis key terms of the neighbour coordinates (olc_tissue_axis)
-        olc_u32 kx[3], ky[3], kz[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            kx[d] = olc_tissue_axis(cx + d - 1, 0);
-            ky[d] = olc_tissue_axis(cy + d - 1, 1);
-            kz[d] = olc_tissue_axis(cz + d - 1, 2);
-        }
-        int nb = 0;
-        for (int dz = -1; dz <= 1; ++dz) {
-            const int nz = cz + dz;
-            if (nz < 0 || nz >= c.tdims[2]) continue;
-            for (int dy = -1; dy <= 1; ++dy) {
-                const int ny = cy + dy;
-                if (ny < 0 || ny >= c.tdims[1]) continue;
-                for (int dx = -1; dx <= 1; ++dx) {
-                    const int nx = cx + dx;
-                    if (nx < 0 || nx >= c.tdims[0]) continue;
-                    const uint2 rg = __ldg(ranges + (kx[dx + 1] | ky[dy + 1] | kz[dz + 1]));
-                    if (rg.y > rg.x) s_bins[nb++][t] = rg;
-                }
-            }
-        }
-        float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-        // the next candidate's record is requested before this one is used
-        int b = 0;
-        olc_u32 j = 0, end = 0;
-        float4 q = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-        if (nb > 0) {
-            const uint2 r = s_bins[0][t];
-            j = r.x;
-            end = r.y;
-            q = __ldg(posr + j);
-        }
-        while (b < nb) {
-            olc_u32 jn = j + 1, en = end;
-            int bn = b;
-            if (jn == en) {
-                if (++bn < nb) {
-                    const uint2 r = s_bins[bn][t];
-                    jn = r.x;
-                    en = r.y;
-                }
-            }
-            const float4 qn = bn < nb ? __ldg(posr + jn) : q;
-            contact_pair(p, q, i, j, c, fx, fy, fz);
-            j = jn;
-            end = en;
-            b = bn;
-            q = qn;
-        }
-        float mx = __fmul_rn(fx, md), my = __fmul_rn(fy, md), mz = __fmul_rn(fz, md);
-        const float len = sqrtf(__fadd_rn(__fadd_rn(__fmul_rn(mx, mx), __fmul_rn(my, my)), __fmul_rn(mz, mz)));
-        if (len > c.max_disp) {
-            const float sc = __fdiv_rn(c.max_disp, len);
-            mx = __fmul_rn(mx, sc);
-            my = __fmul_rn(my, sc);
-            mz = __fmul_rn(mz, sc);
-        }
-        xo[i] = fminf(fmaxf(__fadd_rn(p.x, mx), c.lo[0]), c.hi[0]);
-        yo[i] = fminf(fmaxf(__fadd_rn(p.y, my), c.lo[1]), c.hi[1]);
-        zo[i] = fminf(fmaxf(__fadd_rn(p.z, mz), c.lo[2]), c.hi[2]);
+    for (olc_u32 first = blockIdx.x * CF_THREADS; first < n; first += gridDim.x * CF_THREADS) {
+        const olc_u32 i = first + threadIdx.x;
+        const float4 p = i < n ? posr[i] : make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+        const bool active = !(p.w < 0.0f);  // else dead this step: no move, no force
+        const float3 f = contact_force_thread<CF_THREADS, CF_HITS>(
+            posr, n, p, i, active, contact_bin(p, c.tvs, c.tdims), c.stiffness, ranges, c.tdims, s_runs, s_hits);
+        if (active) contact_move(p, f, i, c, c.lo, c.hi, xo, yo, zo);
     }
 }
 
-// The two walks (olc.h OLC_CONTACT_*): bit-identical, chosen per handle by
-// measurement (OlcTuning.contact_variant).  On the 1 M-agent scale workload
-// the flat walk took 0.92 ms per step over 200 steps against 1.04 for the
-// nested loops; sparser or denser populations can order them the other way.
+// The same sum by contact_force_warp.
+constexpr int CW_THREADS = 64, CW_AGENTS = 8, CW_CAP = 128, CW_BLOCK = CW_AGENTS * (CW_THREADS / 32);
+__global__ void __launch_bounds__(CW_THREADS) k_contact_warp(const float4* __restrict__ posr,
+                                                            const uint2* __restrict__ ranges, const olc_u32* n_dev,
+                                                            olc_u32 n_host, const __grid_constant__ ContactDev c,
+                                                            float* __restrict__ xo, float* __restrict__ yo,
+                                                            float* __restrict__ zo) {
+    __shared__ ContactWarp<CW_AGENTS, CW_CAP> s_warp[CW_THREADS / 32];
+    const olc_u32 n = n_dev ? *n_dev : n_host;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (olc_u32 first = blockIdx.x * CW_BLOCK; first < n; first += gridDim.x * CW_BLOCK) {
+        const olc_u32 base = first + warp * CW_AGENTS, i = base + lane;
+        const float4 p = lane < CW_AGENTS && i < n ? posr[i] : make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+        const bool active = !(p.w < 0.0f);
+        const float3 f = contact_force_warp(posr, base, p, contact_bin(p, c.tvs, c.tdims), active, c.stiffness,
+                                            ranges, c.tdims, s_warp[warp]);
+        if (active) contact_move(p, f, i, c, c.lo, c.hi, xo, yo, zo);
+    }
+}
+
+// The flat walk (OLC_CONTACT_FLAT) is a warp per eight agents up to CW_MAX rows of
+// capacity, a thread per agent above, where it fills the SMs: us with a warp and with
+// a thread at 10,000 rows 13 and 26, 40,000 25 and 35 (22 and 21 if sparse, 35 and
+// 51 if dense), 80,000 38 and 39, 120,000 52 and 45, 1 M 374 and 274.  The nested
+// loops of k_contact are the other choice (OlcTuning.contact_variant); all give the
+// same bits.
+constexpr olc_u32 CW_MAX = 49152;
 void launch_contact(const float4* posr, const olc_u32* ranges, const olc_u32* n_dev, olc_u32 n_host,
                     olc_u32 n_cap, const ContactDev& c, float* x, float* y, float* z, cudaStream_t s, int variant,
                     olc_u32 n_table) {
     if (variant != OLC_CONTACT_NESTED) {
+        const uint2* rg = reinterpret_cast<const uint2*>(ranges);
+        if (n_cap <= CW_MAX) {
+            const olc_u32 blocks = n_cap == 0 ? 1 : (n_cap + CW_BLOCK - 1) / CW_BLOCK;
+            k_contact_warp<<<blocks, CW_THREADS, 0, s>>>(posr, rg, n_dev, n_host, c, x, y, z);
+            return;
+        }
         olc_u32 blocks = (n_cap + CF_THREADS - 1) / CF_THREADS;
-        if (blocks == 0) blocks = 1;
-        if (blocks > 148 * 16) blocks = 148 * 16;
-        k_contact_flat<<<blocks, CF_THREADS, 0, s>>>(posr, reinterpret_cast<const uint2*>(ranges), n_dev, n_host, c,
-                                                      x, y, z);
+        if (blocks > 148 * 64) blocks = 148 * 64;
+        k_contact_flat<<<blocks, CF_THREADS, 0, s>>>(posr, rg, n_dev, n_host, c, x, y, z);
         return;
     }
     olc_u32 blocks = (n_cap + 255) / 256;
