@@ -612,8 +612,9 @@ int olc_stage_keys(const float* x_dev, const float* y_dev, const float* z_dev,
                    uint32_t* keys_dev, void* stream);
 
 /* Stable LSD radix sort of (key, value) pairs on the low `key_bits` bits
- * (onesweep: one upfront digit histogram, then one decoupled-look-back pass
- * per 8-bit digit).  Replaces the counting sort of template.wgsl:165-343.
+ * (up to 65,536 rows in one launch of one thread-block cluster, else onesweep:
+ * one upfront digit histogram, then one decoupled-look-back pass per 8-bit
+ * digit).  Replaces the counting sort of template.wgsl:165-343.
  * vals_in_dev == NULL means values 0..n-1.  Scratch is caller memory of at
  * least olc_sort_scratch_bytes(n, key_bits) bytes, 256-byte aligned.  The
  * sort's status word is the uint32 at byte olc_sort_status_offset() of the

@@ -63,7 +63,9 @@ __global__ void __launch_bounds__(256) k_keys_batch(const float* __restrict__ x,
     __shared__ olc_u32 sh[MAX_PASSES][RADIX];
     __shared__ olc_u32 s_dead;
     const olc_u32 n = olc_total_rows(counters);
-    for (int i = threadIdx.x; i < MAX_PASSES * RADIX; i += blockDim.x) (&sh[0][0])[i] = 0u;
+    if (hist) {
+        for (int i = threadIdx.x; i < MAX_PASSES * RADIX; i += blockDim.x) (&sh[0][0])[i] = 0u;
+    }
     if (threadIdx.x == 0) s_dead = 0u;
     __syncthreads();
     olc_u32 my_dead = 0;
@@ -81,14 +83,16 @@ __global__ void __launch_bounds__(256) k_keys_batch(const float* __restrict__ x,
             k = (s << shift) | olc_tissue_key(cx, cy, cz);
         }
         keys[i] = k;
-        hist_add_b(sh, k, passes);
+        if (hist) hist_add_b(sh, k, passes);
     }
     for (int o = 16; o > 0; o >>= 1) my_dead += __shfl_xor_sync(0xffffffffu, my_dead, o);
     if ((threadIdx.x & 31) == 0 && my_dead) atomicAdd(&s_dead, my_dead);
     __syncthreads();
-    for (int i = threadIdx.x; i < passes * RADIX; i += blockDim.x) {
-        olc_u32 v = (&sh[0][0])[i];
-        if (v) atomicAdd(hist + i, v);
+    if (hist) {
+        for (int i = threadIdx.x; i < passes * RADIX; i += blockDim.x) {
+            olc_u32 v = (&sh[0][0])[i];
+            if (v) atomicAdd(hist + i, v);
+        }
     }
     if (threadIdx.x == 0 && s_dead) atomicAdd(dead_ctr, s_dead);
 }

@@ -1,5 +1,5 @@
-// Spatial grid: bin keys, stable LSD radix sort (onesweep), bin table, payload
-// permute.  Replaces the reference's counting sort
+// Spatial grid: bin keys, stable LSD radix sort (one cluster for few rows, else
+// onesweep), bin table, payload permute.  Replaces the reference's counting sort
 // (framework/src/oncolytica/gpu/compiler/template.wgsl:152-343:
 // Kernel_ClearVoxels, Kernel_CountAndOffset, Kernel_Scan_L0/L1/L2,
 // Kernel_AddBack_L1/L0, Kernel_Scatter, Kernel_UpdateState).
@@ -11,6 +11,7 @@
 #include "olc_internal.h"
 
 #include <algorithm>
+#include <atomic>
 
 namespace olc {
 
@@ -132,6 +133,23 @@ __device__ __forceinline__ olc_u32 block_excl_scan256(olc_u32 v, olc_u32* s_w) {
     return r;
 }
 
+// Commits the previous step's row count and this sort's compaction.
+__device__ __forceinline__ void commit_rows(olc_u32* counters, olc_u32 capacity) {
+    olc_u32 rows = olc_total_rows(counters);
+    if (rows > capacity) rows = capacity;
+    olc_u32 dead = counters[OLC_CTR_DEAD_TMP];
+    counters[OLC_CTR_ROWS] = rows;
+    counters[OLC_CTR_N] = rows - dead;
+    *reinterpret_cast<unsigned long long*>(counters + OLC_CTR_AGENT_STEPS) += (unsigned long long)(rows - dead);
+    counters[OLC_CTR_DEAD] = dead;
+    counters[OLC_CTR_DEAD_TMP] = 0u;
+    counters[OLC_CTR_FIELD_STEP] += 1u;
+    for (int j = 0; j < OLC_MAX_RULE_KERNELS; ++j) {
+        counters[OLC_CTR_BIRTHS + j] = 0u;
+        counters[OLC_CTR_RULE_TILE + j] = 0u;
+    }
+}
+
 __global__ void __launch_bounds__(256) k_scan_hist(const olc_u32* __restrict__ hist, olc_u32* __restrict__ base,
                                                    int passes, olc_u32* tile_ctrs, olc_u32* counters,
                                                    olc_u32 capacity) {
@@ -142,20 +160,7 @@ __global__ void __launch_bounds__(256) k_scan_hist(const olc_u32* __restrict__ h
     }
     if (threadIdx.x < MAX_PASSES) tile_ctrs[threadIdx.x] = 0u;
     if (counters && threadIdx.x == 0) {
-        // Commit the previous step's row count and this sort's compaction.
-        olc_u32 rows = olc_total_rows(counters);
-        if (rows > capacity) rows = capacity;
-        olc_u32 dead = counters[OLC_CTR_DEAD_TMP];
-        counters[OLC_CTR_ROWS] = rows;
-        counters[OLC_CTR_N] = rows - dead;
-        *reinterpret_cast<unsigned long long*>(counters + OLC_CTR_AGENT_STEPS) += (unsigned long long)(rows - dead);
-        counters[OLC_CTR_DEAD] = dead;
-        counters[OLC_CTR_DEAD_TMP] = 0u;
-        counters[OLC_CTR_FIELD_STEP] += 1u;
-        for (int j = 0; j < OLC_MAX_RULE_KERNELS; ++j) {
-            counters[OLC_CTR_BIRTHS + j] = 0u;
-            counters[OLC_CTR_RULE_TILE + j] = 0u;
-        }
+        commit_rows(counters, capacity);
     }
 }
 
@@ -262,6 +267,145 @@ __global__ void __launch_bounds__(SORT_THREADS) k_onesweep(const olc_u32* __rest
             }
         }
         __syncthreads();  // shared tiles are reused by the block's next tile
+    }
+}
+
+// ------------------------------------------------------------------ small sort
+// The whole sort of up to SMALL_SORT_ROWS pairs in one launch, by one cluster of
+// sixteen CTAs that keep the pairs in shared memory.  With so few rows the passes
+// above are a chain of launches and of look-backs over a few tiles; here a pass
+// costs two cluster barriers: one after the CTAs exchanged their digit counts, one
+// after they scattered the pairs to their places in each other's shared memory.
+// Stable: CTA, warp, round and lane follow the row order.
+// us, two memsets, histogram, scan and passes -> this: 10,007 rows of 16 bits
+// 38 -> 13, 20,000 38 -> 15, 65,536 41 -> 27 (43 with eight CTAs of 1,024 threads);
+// 65,535 of 32 bits 66 -> 54.
+constexpr int SMALL_CTAS = 16, SMALL_THREADS = 512, SMALL_WARPS = SMALL_THREADS / 32;
+constexpr int SMALL_IPT = 8;  // rows per thread at most
+
+__device__ __forceinline__ olc_u32 cluster_addr(const void* p, olc_u32 cta) {
+    olc_u32 r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((olc_u32)__cvta_generic_to_shared(p)), "r"(cta));
+    return r;
+}
+__device__ __forceinline__ void cluster_store(olc_u32 addr, olc_u32 v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// `per_cap` rows of each CTA fit its dynamic shared memory (two buffers of keys
+// and values).  With counters the rows are the step's (olc_total_rows) and the
+// counts are committed as k_scan_hist does.
+__global__ void __launch_bounds__(SMALL_THREADS) k_sort_small(const olc_u32* __restrict__ kin,
+                                                              const olc_u32* __restrict__ vin, olc_u32* kout,
+                                                              olc_u32* vout, olc_u32 n_host, olc_u32 per_cap,
+                                                              int key_bits, olc_u32* counters, olc_u32 capacity,
+                                                              olc_u32* status) {
+    extern __shared__ olc_u32 s_rows[];  // keys, values, keys, values
+    __shared__ olc_u32 s_whist[SMALL_WARPS][RADIX];
+    __shared__ olc_u32 s_cnt[SMALL_CTAS][RADIX];
+    __shared__ olc_u32 s_base[RADIX];
+    __shared__ olc_u32 s_w[RADIX / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const olc_u32 cta = blockIdx.x;  // the grid is the cluster
+    olc_u32 n = n_host;
+    if (counters)
+        n = min(olc_total_rows(counters), capacity);
+    else if (cta == 0 && tid == 0)
+        *status = 0u;  // nothing waits here
+    n = min(n, per_cap * SMALL_CTAS);
+    const olc_u32 per = (n + SMALL_CTAS - 1) / SMALL_CTAS;
+    const olc_u32 first = min(cta * per, n), mine = min(per, n - first);
+    const int ipt = (int)((per + SMALL_THREADS - 1) / SMALL_THREADS);
+    const olc_u32 wbase = (olc_u32)(warp * 32 * ipt + lane), lt_mask = (1u << lane) - 1u;
+    olc_u32 *ck = s_rows, *nk = s_rows + 2 * per_cap;
+    for (olc_u32 i = tid; i < mine; i += SMALL_THREADS) {
+        ck[i] = kin[first + i];
+        ck[per_cap + i] = vin ? vin[first + i] : first + i;
+    }
+    for (int i = tid; i < SMALL_WARPS * RADIX; i += SMALL_THREADS) (&s_whist[0][0])[i] = 0u;
+    __syncthreads();
+    const int passes = (key_bits + 7) / 8;
+    for (int p = 0; p < passes; ++p) {
+        const int shift = 8 * p;
+        const olc_u32 mask = (1u << min(8, key_bits - shift)) - 1u;
+        olc_u32 ranks[SMALL_IPT];
+#pragma unroll
+        for (int j = 0; j < SMALL_IPT; ++j) {
+            if (j >= ipt) break;
+            const olc_u32 i = wbase + 32u * j;
+            const bool valid = i < mine;
+            const olc_u32 d = valid ? (ck[i] >> shift) & mask : 0x100u + (olc_u32)lane;
+            const olc_u32 peers = __match_any_sync(0xffffffffu, d);
+            const olc_u32 before = __popc(peers & lt_mask);
+            const olc_u32 b = valid ? s_whist[warp][d] : 0u;
+            __syncwarp();
+            if (valid && before == 0u) s_whist[warp][d] = b + (olc_u32)__popc(peers);
+            __syncwarp();
+            ranks[j] = b + before;
+        }
+        __syncthreads();
+        if (tid < RADIX) {  // thread == digit: places of the warps' rows, and the CTA's count to all CTAs
+            olc_u32 total = 0;
+#pragma unroll
+            for (int w = 0; w < SMALL_WARPS; ++w) {
+                const olc_u32 c = s_whist[w][tid];
+                s_whist[w][tid] = total;
+                total += c;
+            }
+#pragma unroll
+            for (int r = 0; r < SMALL_CTAS; ++r) cluster_store(cluster_addr(&s_cnt[cta][tid], r), total);
+        }
+        cluster_barrier();
+        if (p == 0 && counters && cta == 0 && tid == 0) commit_rows(counters, capacity);  // all CTAs have read them
+        olc_u32 before = 0, incl = 0, all = 0;
+        if (tid < RADIX) {
+#pragma unroll
+            for (int r = 0; r < SMALL_CTAS; ++r) {
+                const olc_u32 c = s_cnt[r][tid];
+                if (r < (int)cta) before += c;
+                all += c;
+            }
+            incl = all;
+            for (int o = 1; o < 32; o <<= 1) {
+                const olc_u32 t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (lane == 31) s_w[warp] = incl;
+        }
+        __syncthreads();
+        if (tid < RADIX) {
+            for (int w = 0; w < warp; ++w) before += s_w[w];
+            s_base[tid] = before + incl - all;
+        }
+        __syncthreads();
+        const bool last = p + 1 == passes;
+#pragma unroll
+        for (int j = 0; j < SMALL_IPT; ++j) {
+            if (j >= ipt) break;
+            const olc_u32 i = wbase + 32u * j;
+            if (i < mine) {
+                const olc_u32 k = ck[i], v = ck[per_cap + i], d = (k >> shift) & mask;
+                const olc_u32 o = s_base[d] + s_whist[warp][d] + ranks[j];
+                if (last) {
+                    kout[o] = k;
+                    vout[o] = v;
+                } else {
+                    const olc_u32 r = o / per, a = cluster_addr(nk + (o - r * per), r);
+                    cluster_store(a, k);
+                    cluster_store(a + 4u * per_cap, v);
+                }
+            }
+        }
+        if (last) break;
+        cluster_barrier();
+        for (int i = tid; i < SMALL_WARPS * RADIX; i += SMALL_THREADS) (&s_whist[0][0])[i] = 0u;
+        olc_u32* t = ck;
+        ck = nk;
+        nk = t;
+        __syncthreads();
     }
 }
 
@@ -389,9 +533,60 @@ __global__ void __launch_bounds__(256) k_clear_lookback(uint4* lookback, const o
             lookback[p * stride + i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
+static_assert(SMALL_CTAS * SMALL_THREADS * SMALL_IPT >= SMALL_SORT_ROWS, "rows of the small sort");
+
+static cudaLaunchConfig_t small_sort_config(olc_u32 per_cap, cudaLaunchAttribute* attr, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(SMALL_CTAS);
+    cfg.blockDim = dim3(SMALL_THREADS);
+    cfg.dynamicSmemBytes = (size_t)per_cap * 16;
+    cfg.stream = s;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = SMALL_CTAS;
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Whether a sort of n_cap rows of capacity takes k_sort_small: up to the rows its
+// shared memory holds (it is the faster one to there), on a device that can place a
+// cluster of its size (asked once per device).
+bool sort_is_small(olc_u32 n_cap) {
+    if (n_cap > SMALL_SORT_ROWS) return false;
+    static std::atomic<int> can[32];  // 0: not asked yet, 1: yes, 2: no
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 32) return false;
+    int c = can[dev].load(std::memory_order_relaxed);
+    if (c == 0) {
+        const olc_u32 per_cap = SMALL_SORT_ROWS / SMALL_CTAS;
+        cudaLaunchAttribute attr[1];
+        const cudaLaunchConfig_t cfg = small_sort_config(per_cap, attr, nullptr);
+        int clusters = 0;
+        const bool ok = cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(per_cap * 16)) == cudaSuccess &&
+                        cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                            cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&clusters, k_sort_small, &cfg) == cudaSuccess && clusters > 0;
+        if (!ok) cudaGetLastError();
+        c = ok ? 1 : 2;
+        can[dev].store(c, std::memory_order_relaxed);
+    }
+    return c == 1;
+}
+
 void run_sort(const olc_u32* kin, const olc_u32* vin, olc_u32* kout, olc_u32* vout, const olc_u32* n_dev,
               olc_u32 n_host, olc_u32 n_cap, int key_bits, const SortScratch& sc, bool hist_ready,
               olc_u32* counters, olc_u32 capacity, cudaStream_t s) {
+    if (sort_is_small(n_cap)) {
+        const olc_u32 per_cap = (n_cap + SMALL_CTAS - 1) / SMALL_CTAS;
+        cudaLaunchAttribute attr[1];
+        const cudaLaunchConfig_t cfg = small_sort_config(per_cap, attr, s);
+        cudaLaunchKernelEx(&cfg, k_sort_small, kin, vin, kout, vout, n_host, per_cap, key_bits, counters, capacity,
+                           sc.status);
+        return;
+    }
     const int passes = (key_bits + 7) / 8;
     const size_t tiles = (n_cap + SORT_TILE - 1) / SORT_TILE ? (n_cap + SORT_TILE - 1) / SORT_TILE : 1;
     // with the row count on the device (committed by the scan below), only the

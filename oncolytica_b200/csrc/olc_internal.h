@@ -73,6 +73,10 @@ struct SortScratch {
     olc_u32* valt;      // n
     size_t lookback_words;
 };
+// Sorts of up to SMALL_SORT_ROWS rows of capacity take one launch and use no
+// scratch, nor a histogram (sort_is_small).
+constexpr olc_u32 SMALL_SORT_ROWS = 65536;
+bool sort_is_small(olc_u32 n_cap);
 bool carve_sort_scratch(void* base, size_t bytes, olc_u32 n_cap, int key_bits, SortScratch* out);
 void run_sort(const olc_u32* kin, const olc_u32* vin, olc_u32* kout, olc_u32* vout,
               const olc_u32* n_dev, olc_u32 n_host, olc_u32 n_cap, int key_bits,

@@ -397,10 +397,12 @@ int step_once(OlcSim* s, int collect, cudaStream_t st) {
     // 2. grid + compaction
     const int passes = (s->key_bits + 7) / 8;
     const int ac = s->agent_cur;
-    OLC_TRY(check(s, cudaMemsetAsync(s->sc.hist, 0, MAX_PASSES * RADIX * 4, st), "memset hist"));
+    const bool small = sort_is_small(cap);  // needs no histogram
+    olc_u32* const hist = small ? nullptr : s->sc.hist;
+    if (hist) OLC_TRY(check(s, cudaMemsetAsync(hist, 0, MAX_PASSES * RADIX * 4, st), "memset hist"));
     launch_keys(static_cast<const float*>(s->col[ac][0]), static_cast<const float*>(s->col[ac][1]),
                 static_cast<const float*>(s->col[ac][2]), s->life, nullptr, 0, s->counters, cap, s->bins,
-                s->keys_in, s->sc.hist, passes, s->counters + OLC_CTR_DEAD_TMP, st);
+                s->keys_in, hist, passes, s->counters + OLC_CTR_DEAD_TMP, st);
     run_sort(s->keys_in, nullptr, s->keys, s->vals, s->counters + OLC_CTR_ROWS, 0, cap, s->key_bits, s->sc,
              true, s->counters, cap, st);
     OLC_TRY(check(s, cudaMemsetAsync(s->ranges, 0, (size_t)s->n_table * 8, st), "memset ranges"));
@@ -419,7 +421,7 @@ int step_once(OlcSim* s, int collect, cudaStream_t st) {
     pa.life = s->life;
     launch_permute(s->vals, s->counters, cap, pa, st);
     s->agent_cur = 1 - ac;
-    launches += 4 + (uint64_t)passes;  // keys, scan, passes, bin table, permute
+    launches += small ? 4 : 4 + (uint64_t)passes;  // keys, sort or scan and passes, bin table, permute
     // 3a. tissue rules, then chemistry rules (one thread per voxel; each reads
     // the state before it and writes the other buffer)
     for (size_t k = 0; k < s->funcs.size(); ++k) {
@@ -602,10 +604,12 @@ int step_once_batch(OlcSim* s, int collect, cudaStream_t st) {
     const int passes = (s->key_bits + 7) / 8;
     const int ac = s->agent_cur;
     const int sim_col = (int)s->caps.n_agent_fields - 1;
-    OLC_TRY(check(s, cudaMemsetAsync(s->sc.hist, 0, MAX_PASSES * RADIX * 4, st), "memset hist"));
+    const bool small = sort_is_small(cap);  // needs no histogram
+    olc_u32* const hist = small ? nullptr : s->sc.hist;
+    if (hist) OLC_TRY(check(s, cudaMemsetAsync(hist, 0, MAX_PASSES * RADIX * 4, st), "memset hist"));
     launch_keys_batch(B, static_cast<const float*>(s->col[ac][0]), static_cast<const float*>(s->col[ac][1]),
                       static_cast<const float*>(s->col[ac][2]), static_cast<const olc_u32*>(s->col[ac][sim_col]),
-                      s->life, s->counters, cap, s->keys_in, s->sc.hist, passes, s->counters + OLC_CTR_DEAD_TMP, st);
+                      s->life, s->counters, cap, s->keys_in, hist, passes, s->counters + OLC_CTR_DEAD_TMP, st);
     run_sort(s->keys_in, nullptr, s->keys, s->vals, s->counters + OLC_CTR_ROWS, 0, cap, s->key_bits, s->sc, true,
              s->counters, cap, st);
     if (s->pool) {
@@ -628,7 +632,7 @@ int step_once_batch(OlcSim* s, int collect, cudaStream_t st) {
     pa.life = s->life;
     launch_permute(s->vals, s->counters, cap, pa, st);
     s->agent_cur = 1 - ac;
-    launches += 4 + (uint64_t)passes;
+    launches += small ? 4 : 4 + (uint64_t)passes;
     // 3a. chemistry rules over every member (a CTA per field tile), each
     // iteration writing the members' other buffers, whose parity then flips
     for (size_t k = 0; k < s->funcs.size(); ++k) {
@@ -2451,7 +2455,7 @@ int olc_stage_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* kou
                     "olc_stage_sort_pairs: scratch too small or not 256-byte aligned (need " +
                         std::to_string(sort_scratch_bytes(n, key_bits)) + " bytes)");
     cudaStream_t st = as_stream(stream);
-    cudaMemsetAsync(sc.status, 0, 4, st);
+    if (!sort_is_small(n)) cudaMemsetAsync(sc.status, 0, 4, st);
     run_sort(kin, vin, kout, vout, nullptr, n, n, key_bits, sc, false, nullptr, 0, st);
     return cuda_status(cudaGetLastError(), "olc_stage_sort_pairs");
 }

@@ -1,0 +1,41 @@
+"""The sort that takes one launch, and the first sizes beyond it, against a
+stable sort."""
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from oncolytica_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", ["random", "equal", "descending", "values"])
+@pytest.mark.parametrize("bits", [1, 8, 9, 17, 32])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 8191, 8193, 10007, 65535, 65536, 65537])
+def test_small_sort_is_the_stable_sort(cuda, olc, n, bits, kind):
+    import torch
+
+    rng = np.random.default_rng(n + bits)
+    k = rng.integers(0, 1 << bits, n, dtype=np.uint64).astype(np.uint32)
+    if kind == "equal":
+        k[:] = k[0]
+    if kind == "descending":
+        k = np.sort(k)[::-1].copy()
+    v = rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32) if kind == "values" else None
+    order = np.argsort(k, kind="stable")
+    dev = lambda a: torch.from_numpy(a.view(np.int32).copy()).to(cuda)  # noqa: E731
+    kin, kout, vout = dev(k), dev(np.zeros_like(k)), dev(np.zeros_like(k))
+    vin = dev(v) if v is not None else None
+    nbytes = olc.olc_sort_scratch_bytes(n, bits)
+    scratch = torch.full((nbytes,), 255, dtype=torch.uint8, device=cuda)
+    ptr = lambda t: C.c_void_p(t.data_ptr()) if t is not None else None  # noqa: E731
+    _lib.check(olc.olc_stage_sort_pairs(ptr(kin), ptr(vin), ptr(kout), ptr(vout), n, bits, ptr(scratch), nbytes, None))
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(kout.cpu().numpy().view(np.uint32), k[order])
+    np.testing.assert_array_equal(vout.cpu().numpy().view(np.uint32), v[order] if v is not None else order)
+    np.testing.assert_array_equal(kin.cpu().numpy().view(np.uint32), k)
+    at = olc.olc_sort_status_offset()
+    assert scratch[at:at + 4].cpu().numpy().view(np.uint32)[0] == 0
