@@ -39,3 +39,29 @@ def test_small_sort_is_the_stable_sort(cuda, olc, n, bits, kind):
     np.testing.assert_array_equal(kin.cpu().numpy().view(np.uint32), k)
     at = olc.olc_sort_status_offset()
     assert scratch[at:at + 4].cpu().numpy().view(np.uint32)[0] == 0
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("bits", [7, 16, 17, 32])
+@pytest.mark.parametrize("n", [65537, 65552, 139265])
+def test_sort_by_passes_counts_every_key(cuda, olc, n, bits, offset):
+    """Keys at and off a 16-byte boundary, with a last thread's share that is not
+    full, in runs of equal digits and in none."""
+    import torch
+
+    rng = np.random.default_rng(n + bits)
+    k = np.sort(rng.integers(0, 1 << bits, n, dtype=np.uint64).astype(np.uint32))
+    moved = rng.random(n) < 0.2
+    k[moved] = rng.integers(0, 1 << bits, int(moved.sum()), dtype=np.uint64).astype(np.uint32)
+    order = np.argsort(k, kind="stable")
+    room = torch.zeros(n + 4, dtype=torch.int32, device=cuda)
+    kin = room[offset:offset + n]
+    kin.copy_(torch.from_numpy(k.view(np.int32).copy()))
+    kout, vout = (torch.zeros(n, dtype=torch.int32, device=cuda) for _ in range(2))
+    nbytes = olc.olc_sort_scratch_bytes(n, bits)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=cuda)
+    ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    _lib.check(olc.olc_stage_sort_pairs(ptr(kin), None, ptr(kout), ptr(vout), n, bits, ptr(scratch), nbytes, None))
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(kout.cpu().numpy().view(np.uint32), k[order])
+    np.testing.assert_array_equal(vout.cpu().numpy().view(np.uint32), order)
