@@ -74,8 +74,8 @@ def parse() -> argparse.Namespace:
     ap.add_argument("--contact", default="auto", choices=["auto", "flat", "nested"],
                     help="contact walk of the scale workload (auto: the tuner's choice)")
     ap.add_argument("--grid", type=int, default=256, help="field edge of --workload stencil")
-    ap.add_argument("--stencil-pair", default="0,1024,512",
-                    help="CTA sizes of the two-substep pass timed by --workload stencil (0: one substep per pass)")
+    ap.add_argument("--stencil-pair", default="0,256",
+                    help="passes timed by --workload stencil (0: one substep per pass, 256: two)")
     ap.add_argument("--encodings", default="value,deficit,offset3",
                     help="16-bit element encodings timed by --workload stencil")
     ap.add_argument("--l2-keep", default="0,30,45,60",
@@ -469,8 +469,8 @@ def run_b200(args) -> None:
         single_ms = (tuning.get("measured_ms", {}).get("substeps", {})
                      .get(f"{t['stencil_tile'][0]}x{t['stencil_tile'][1]}", sub_ms * sum(subs)) / sum(subs))
         launch_ms = max(1e-6, (sub_ms * sum(subs) - n_single * single_ms) / max(1, n_pairs))
-        kernel = f"k_substep_pair<{pair[0]}> (two 7-point FTCS substeps per pass, FP32, TMA plane ring)"
-        traffic = read_traffic("k_substep_pair", nvox)
+        kernel = "k_march2 (two 7-point FTCS substeps per pass, FP32, TMA plane ring)"
+        traffic = read_traffic("k_march2", nvox)
     else:
         launch_ms = sub_ms
         kernel = "k_substep_x4 (7-point FTCS, FP32, 4-wide rows, TMA tiles)"

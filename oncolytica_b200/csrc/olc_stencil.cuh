@@ -182,21 +182,4 @@ __device__ __forceinline__ void stencil_update8_enc(float xl, float xr, const fl
     }
 }
 
-// Eight consecutive x voxels (four pairs): centre row c, rows ym/yp, planes
-// zm/zp, and the neighbours xl/xr left and right of the group.
-__device__ __forceinline__ void stencil_update8(float xl, float xr, const float (&c)[8], const float (&ym)[8],
-                                                const float (&yp)[8], const float (&zm)[8], const float (&zp)[8],
-                                                float r, float inv_decay, float (&out)[8]) {
-    const f32x2 r2 = pk2(r, r), id2 = pk2(inv_decay, inv_decay);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int e = 2 * k;
-        const float2 v = stencil_update2(pk2(k == 0 ? xl : c[e - 1], c[e]), pk2(c[e + 1], k == 3 ? xr : c[e + 2]),
-                                         pk2(ym[e], ym[e + 1]), pk2(yp[e], yp[e + 1]), pk2(zm[e], zm[e + 1]),
-                                         pk2(zp[e], zp[e + 1]), pk2(c[e], c[e + 1]), r2, id2);
-        out[e] = v.x;
-        out[e + 1] = v.y;
-    }
-}
-
 }  // namespace olc
