@@ -75,11 +75,12 @@ def parse() -> argparse.Namespace:
                     help="contact walk of the scale workload (auto: the tuner's choice)")
     ap.add_argument("--grid", type=int, default=256, help="field edge of --workload stencil")
     ap.add_argument("--stencil-pair", default="0,256",
-                    help="passes timed by --workload stencil (0: one substep per pass, 256: two)")
+                    help="passes timed by --workload stencil (0: the library's choice, 256: two substeps each)")
     ap.add_argument("--encodings", default="value,deficit,offset3",
                     help="16-bit element encodings timed by --workload stencil")
     ap.add_argument("--l2-keep", default="0,30,45,60",
-                    help="shares (%%) of the FP32 field kept in L2 timed by --workload stencil (one substep per pass)")
+                    help="shares (%%) of the FP32 field kept in L2 timed by --workload stencil (one substep per pass; "
+                         "0: the library's choice)")
     return ap.parse_args()
 
 
@@ -456,25 +457,26 @@ def run_b200(args) -> None:
     peaks = measured_peaks()
     sub_ms = prof["ms_substeps"] / max(1, prof["substep_launches"])  # per substep (a pair counts two)
     alg_bytes = 8 * nvox  # read 4 B + write 4 B per voxel and launch (FP32)
-    pair = tuple((tuning.get("tuning") or {}).get("stencil_pair", (0, 0)))
-    paired = pair[0] > 0 and autotune.pair_applies(pair[0], spec.field_dims)
+    t = tuning.get("tuning") or {}
+    paired = autotune.takes_pairs(t, spec.field_dims)
     if paired:
         # two substeps per launch: the odd substep of each field is a single
         # pass, so a pair launch takes the fields' time less those singles,
-        # timed at the single-pass time per substep the tuner measured
+        # timed at the best time per substep the tuner measured on a tile
+        # shape, which takes one pass each (the default shape leaves the choice
+        # to the library)
         subs = [S for S in (spec.S_o2, spec.S_drug) if S]
         n_pairs = sum(S // 2 for S in subs)
         n_single = sum(S % 2 for S in subs)
-        t = tuning["tuning"]
-        single_ms = (tuning.get("measured_ms", {}).get("substeps", {})
-                     .get(f"{t['stencil_tile'][0]}x{t['stencil_tile'][1]}", sub_ms * sum(subs)) / sum(subs))
+        shapes = {k: v for k, v in tuning.get("measured_ms", {}).get("substeps", {}).items() if k != "8x8"}
+        single_ms = min(shapes.values(), default=sub_ms * sum(subs)) / sum(subs)
         launch_ms = max(1e-6, (sub_ms * sum(subs) - n_single * single_ms) / max(1, n_pairs))
         kernel = "k_march2 (two 7-point FTCS substeps per pass, FP32, TMA plane ring)"
         traffic = read_traffic("k_march2", nvox)
     else:
         launch_ms = sub_ms
         kernel = "k_substep_x4 (7-point FTCS, FP32, 4-wide rows, TMA tiles)"
-        keep = (tuning.get("tuning") or {}).get("l2_keep_pct", 0)
+        keep = t.get("l2_keep_pct", 0)
         traffic = read_traffic("k_substep_x4_l2slab" if keep else "k_substep_x4_scale", nvox)
     achieved = alg_bytes / (launch_ms / 1e3) / 1e9
     steps_done = max(1, prof["steps"])
