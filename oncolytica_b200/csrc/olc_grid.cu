@@ -318,7 +318,8 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) k_onesweep(const olc_u32* __r
 // sixteen CTAs that keep the pairs in shared memory.  With so few rows the passes
 // above are a chain of launches and of look-backs over a few tiles; here a pass
 // costs two cluster barriers: one after the CTAs exchanged their digit counts, one
-// after they scattered the pairs to their places in each other's shared memory.
+// after they scattered the pairs to their places in each other's shared memory; a
+// third, hidden behind the first ranking, sees to it that all CTAs have started.
 // Stable: CTA, warp, round and lane follow the row order.
 // us, two memsets, histogram, scan and passes -> this: 10,007 rows of 16 bits
 // 38 -> 13, 20,000 38 -> 15, 65,536 41 -> 27 (43 with eight CTAs of 1,024 threads);
@@ -334,8 +335,15 @@ __device__ __forceinline__ olc_u32 cluster_addr(const void* p, olc_u32 cta) {
 __device__ __forceinline__ void cluster_store(olc_u32 addr, olc_u32 v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
+__device__ __forceinline__ void cluster_arrive() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 
 // `per_cap` rows of each CTA fit its dynamic shared memory (two buffers of keys
@@ -353,6 +361,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_sort_small(const olc_u32* __r
     __shared__ olc_u32 s_w[RADIX / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const olc_u32 cta = blockIdx.x;  // the grid is the cluster
+    cluster_arrive();  // waited for before the first store to another CTA
     olc_u32 n = n_host;
     if (counters)
         n = min(olc_total_rows(counters), capacity);
@@ -389,6 +398,8 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_sort_small(const olc_u32* __r
             __syncwarp();
             ranks[j] = b + before;
         }
+        // another CTA's shared memory may be written only once that CTA runs
+        if (p == 0) cluster_wait();
         __syncthreads();
         if (tid < RADIX) {  // thread == digit: places of the warps' rows, and the CTA's count to all CTAs
             olc_u32 total = 0;

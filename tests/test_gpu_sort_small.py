@@ -65,3 +65,35 @@ def test_sort_by_passes_counts_every_key(cuda, olc, n, bits, offset):
     torch.cuda.synchronize()
     np.testing.assert_array_equal(kout.cpu().numpy().view(np.uint32), k[order])
     np.testing.assert_array_equal(vout.cpu().numpy().view(np.uint32), order)
+
+
+@pytest.mark.parametrize("n", [1, 16, 500, 4096])
+def test_small_sort_among_other_work(cuda, olc, n):
+    """One-pass sorts, back to back on several streams while other kernels hold the
+    SMs: the cluster's CTAs start at different times, and none may write to another
+    before it has started."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    k = rng.integers(0, 256, n, dtype=np.uint64).astype(np.uint32)
+    order = np.argsort(k, kind="stable")
+    kin = torch.from_numpy(k.view(np.int32).copy()).to(cuda)
+    nbytes = olc.olc_sort_scratch_bytes(n, 8)
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    runs = []
+    noise = torch.zeros(1 << 24, device=cuda)
+    torch.cuda.synchronize()
+    for r in range(32):
+        st = streams[r % 4]
+        noise.add_(1.0)  # on the default stream, beside the sorts
+        with torch.cuda.stream(st):
+            out = [torch.full((n,), -1, dtype=torch.int32, device=cuda) for _ in range(2)]
+            scratch = torch.empty(nbytes, dtype=torch.uint8, device=cuda)
+            runs.append((out, scratch))
+            _lib.check(olc.olc_stage_sort_pairs(C.c_void_p(kin.data_ptr()), None, C.c_void_p(out[0].data_ptr()),
+                                                C.c_void_p(out[1].data_ptr()), n, 8, C.c_void_p(scratch.data_ptr()),
+                                                nbytes, C.c_void_p(st.cuda_stream)))
+    torch.cuda.synchronize()
+    for out, _ in runs:
+        np.testing.assert_array_equal(out[0].cpu().numpy().view(np.uint32), k[order])
+        np.testing.assert_array_equal(out[1].cpu().numpy().view(np.uint32), order)
