@@ -97,6 +97,14 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_march2(const __grid_constant
     const int dir = a.down ? -1 : 1;
     const int first = a.down ? z1 + 1 : z0 - 2;
     const int nq = z1 - z0 + 4;
+    // planes first + dir and first + dir (nq - 2) are the intermediate field's
+    // first and last; either may be a face of the grid
+    const int zi0 = first + dir, zi1 = first + dir * (nq - 2);
+    const bool face0 = zi0 == 0 || zi0 == a.nz - 1, face1 = zi1 == 0 || zi1 == a.nz - 1;
+    // Steps below this one compute their intermediate plane.  Planes below it are
+    // loaded, and every one of them is waited for: the block's shared memory goes
+    // to another block when it ends.
+    const int n_full = face1 ? nq - 1 : nq;
     auto issue = [&](int q, int slot) {
         const olc_u32 bar = full0 + 8 * slot;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(S::BYTES) : "memory");
@@ -108,7 +116,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_march2(const __grid_constant
             : "memory");
     };
     if (threadIdx.x == 0)
-        for (int q = 0; q < S::SLOTS && q < nq; ++q) issue(q, q);
+        for (int q = 0; q < S::SLOTS && q < n_full; ++q) issue(q, q);
 
     const int x = x0 + 4 * lx;
     const int yr = cy0 + unit * R;  // the group's first row
@@ -161,8 +169,8 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_march2(const __grid_constant
     const bool face_rows = top || bottom;
 
     // One step: plane q of the input has arrived; intermediate plane q - 1 from
-    // planes q - 2 .. q (ZF: it is the far z face), output plane q - 2 from mz,
-    // mc and it; it replaces mz.
+    // planes q - 2 .. q (ZF: it is the far z face, and plane q is not read), output
+    // plane q - 2 from mz, mc and it; it replaces mz.
     auto step = [&](auto zface, auto odd, int q, float4 (&mz)[R], const float4 (&mc)[R], float& xmz, const float xmc) {
         constexpr bool ZF = decltype(zface)::value;
         constexpr bool ODD = decltype(odd)::value;  // parity of q
@@ -220,10 +228,10 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_march2(const __grid_constant
             }
         }
         ov += ostep;
-        if (EDGE) {
+        if (EDGE && !ZF) {  // no step follows the one of the far z face
             const float v = stencil_update(pc[xoff - 1], pc[xoff + 1], pc[xoff - S::WX], pc[xoff + S::WX], pm[xoff],
                                            pp[xoff], pc[xoff], a.r, a.inv_decay);
-            xmz = (x_face || ZF) ? bval : v;
+            xmz = x_face ? bval : v;
         }
     };
 
@@ -234,17 +242,12 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_march2(const __grid_constant
     // the plane's slot is refilled; false when a plane never arrived
     auto end_step = [&](int q, bool ok) {
         if (__syncthreads_or(!ok)) return false;
-        if (threadIdx.x == 0 && q - 2 + S::SLOTS < nq) {
+        if (threadIdx.x == 0 && q - 2 + S::SLOTS < n_full) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             issue(q - 2 + S::SLOTS, (q - 2) % S::SLOTS);
         }
         return true;
     };
-    // planes first + dir and first + dir (nq - 2) are the intermediate field's
-    // first and last; either may be a face of the grid
-    const int zi0 = first + dir, zi1 = first + dir * (nq - 2);
-    const bool face0 = zi0 == 0 || zi0 == a.nz - 1, face1 = zi1 == 0 || zi1 == a.nz - 1;
-    const int n_full = face1 ? nq - 1 : nq;  // steps below this one compute their intermediate plane
     bool ok = wait_plane(0) && wait_plane(1);
     int q = 2;
 #pragma unroll 1

@@ -71,6 +71,15 @@ def test_two_substeps_per_pass_bit_exact(cuda, olc, dims, substeps, planes):
              tuning=tuning)
 
 
+@pytest.mark.parametrize("planes", [1, 2, 3])
+@pytest.mark.parametrize("dims", [(260, 200, 40), (512, 62, 64)])
+def test_two_substeps_per_pass_in_many_waves(cuda, olc, dims, planes):
+    """Short chunks along z and several tiles along x, in more CTAs than fit at once
+    and pass after pass: a CTA's shared memory goes to the next one as soon as it
+    ends, so no plane may still be on its way into it (the chunks at the far z face)."""
+    _diffuse(cuda, olc, dims, 12, boundary=0.6, tuning=_lib.OlcTuning(8, 8, 0, 16, 256, planes, 0))
+
+
 def test_two_substeps_per_pass_leave_negative_boundaries_to_single_passes(cuda, olc):
     _diffuse(cuda, olc, (64, 40, 20), 4, boundary=-0.25, tuning=_lib.OlcTuning(8, 8, 0, 16, 256, 0, 0))
 
