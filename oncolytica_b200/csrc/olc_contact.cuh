@@ -244,6 +244,7 @@ __device__ __forceinline__ float3 contact_force_warp(const float4* __restrict__ 
     int cnt = 0, beg = 0, end = 0;
     const int own = lane / 3, comp = lane - 3 * own;
     auto drain = [&]() {
+        __syncwarp();  // the lanes' listed pairs are visible to one another
         for (int h = lane; h < cnt; h += 32) {
             const uint2 hit = s.hit[h];
             const float3 v = contact_pair(s.p[hit.y], __ldg(posr + hit.x), base + hit.y, hit.x, stiffness);

@@ -66,3 +66,38 @@ def test_contact_lists_bit_exact(cuda, olc, n, case):
     torch.cuda.synchronize()
     np.testing.assert_array_equal(np.stack([t.cpu().numpy() for t in xyz], axis=1), ref)
 
+
+
+@pytest.mark.parametrize("per_bin", [17, 40, 127, 129])
+@pytest.mark.parametrize("agents", [300, 3000])
+def test_contact_lists_that_fill_in_mid_bin(cuda, olc, agents, per_bin):
+    """Many bins so full that the warps' lists of near pairs fill up again and again,
+    between and within the agents' shares: every pair listed just before must be seen
+    by the lane that computes it."""
+    import torch
+
+    rng = np.random.default_rng(agents + per_bin)
+    dims, vs = (12, 10, 8), 10.0
+    top = np.array(dims) * vs
+    bins = np.stack([rng.integers(0, d, -(-agents // per_bin)) for d in dims], axis=1)
+    pos = (np.repeat(bins, per_bin, axis=0)[:agents] + 0.98 * rng.random((agents, 3))) * vs
+    pos = np.minimum(pos, top - 0.01).astype(np.float32)
+    ks, perm = oracle.sort_pairs(oracle.keys(pos, dims, vs))
+    ranges = oracle.bin_ranges(ks, oracle.tissue_key(*dims)).reshape(-1, 2).copy()
+    posr = np.concatenate([pos[perm], rng.uniform(4.0, 6.0, (agents, 1))], axis=1).astype(np.float32)
+    lo, hi = (0.1, 0.1, 0.1), tuple(float(t) - 0.1 for t in top)
+    ref = oracle.contact(posr, ranges.reshape(-1), dims, vs, 1.0, 10.0, 1.0, 0.1, lo, hi)
+    pr = torch.from_numpy(posr).to(cuda)
+    rg = torch.from_numpy(ranges.astype(np.uint32).view(np.int32).copy()).to(cuda)
+    g = _lib.OlcGeom()
+    g.tissue_dims[:] = dims
+    g.tissue_voxel_size = vs
+    g.chem_voxel_size = 1.0
+    g.domain_hi[:] = tuple(float(t) for t in top)
+    spec = _lib.OlcContact(enabled=1, radius_field=-1, stiffness=1.0, mobility=10.0, max_disp=1.0, margin=0.1)
+    for _ in range(5):
+        xyz = [torch.zeros(agents, device=cuda) for _ in range(3)]
+        ptr = [C.c_void_p(t.data_ptr()) for t in (pr, rg, *xyz)]
+        _lib.check(olc.olc_stage_contact(ptr[0], ptr[1], agents, C.byref(g), C.byref(spec), 0.1, *ptr[2:], None))
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(np.stack([t.cpu().numpy() for t in xyz], axis=1), ref)
