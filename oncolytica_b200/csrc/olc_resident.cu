@@ -76,7 +76,8 @@ struct ResidentF32 {
         if (VEC) {
             asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
                          : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w)
-                         : "l"(w));
+                         : "l"(w)
+                         : "memory");
             return q;
         }
         q.x = olc_ld_relaxed(w);
@@ -89,7 +90,8 @@ struct ResidentF32 {
         olc_u32* w = static_cast<olc_u32*>(f) + v;
         if (VEC) {
             asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(w), "r"(q.x), "r"(q.y), "r"(q.z),
-                         "r"(q.w));
+                         "r"(q.w)
+                         : "memory");
             return;
         }
         olc_st_relaxed(w, q.x);
@@ -148,12 +150,14 @@ struct Resident16 {
         uint2 q;
         asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];"
                      : "=r"(q.x), "=r"(q.y)
-                     : "l"(static_cast<const unsigned short*>(f) + v));
+                     : "l"(static_cast<const unsigned short*>(f) + v)
+                     : "memory");
         return q;
     }
     static __device__ __forceinline__ void store(void* f, olc_u32 v, int, Raw q) {
         asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(static_cast<unsigned short*>(f) + v), "r"(q.x),
-                     "r"(q.y));
+                     "r"(q.y)
+                     : "memory");
     }
     static __device__ __forceinline__ bool ready(Raw q, olc_u32 phase) {
         return (((q.x ^ phase) | (q.y ^ phase)) & PHASE) == 0u;
@@ -207,16 +211,21 @@ struct Resident16 {
 
 __device__ __forceinline__ float4 lds4(olc_u32 p) {
     float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(p));
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(p)
+                 : "memory");
     return v;
 }
 __device__ __forceinline__ void sts4(olc_u32 p, float4 v) {
-    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w));
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
 // One tile per CTA; a thread owns up to K consecutive planes of four voxels of
 // one row, in registers, and shares them with its neighbours through shared
-// memory (two copies of the tile and its ring of one row and one plane).  What
+// memory (two copies of the tile and its ring of one row and one plane).  The same
+// words are reached by plain accesses and by the asm ones above, whose "memory"
+// clobbers keep the compiler from reordering the two.  What
 // bounds it is latency (the exchange, about 0.8 us) and, on larger tiles,
 // instruction issue: the threads' addresses, faces and publications are worked
 // out once, before the substeps.
@@ -372,9 +381,9 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const ResidentArgs a) {
                 float xr = __shfl_down_sync(0xffffffffu, c[k].x, 1);
                 if (WRAP) {
                     asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; @p ld.shared.f32 %0, [%1 + -4]; }"
-                                 : "+f"(xl) : "r"(pc), "r"(need_l));
+                                 : "+f"(xl) : "r"(pc), "r"(need_l) : "memory");
                     asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; @p ld.shared.f32 %0, [%1 + 16]; }"
-                                 : "+f"(xr) : "r"(pc), "r"(need_r));
+                                 : "+f"(xr) : "r"(pc), "r"(need_r) : "memory");
                 }
                 float4 v = update(xl, xr, c[k], lds4(pm), lds4(pp), prev, lds4(pz));
                 if (E::ROUNDS) v = E::round(v, vo, key);
