@@ -229,8 +229,10 @@ __device__ __forceinline__ void t16_tile4(const unsigned short* tile, unsigned s
     const float bf = face_work<ST, EN>(fs.bval);
     const float4 b4 = make_float4(bf, bf, bf, bf);
     const f32x2 r2 = pk2(fs.r, fs.r), id2 = pk2(fs.inv_decay, fs.inv_decay), ds2 = pk2(fs.dec_sub, fs.dec_sub);
-    const olc_u32 sz = (olc_u32)nx * (olc_u32)ny;
-    olc_u32 vi = (olc_u32)z0 * sz + (olc_u32)y * (olc_u32)nx + (olc_u32)x;  // low 32 bits are all the hash takes
+    // half the own group's voxel index (rows are a multiple of 8 voxels): the hash takes
+    // its low 32 bits, one more than the voxel index's
+    const olc_u32 pair_y = (olc_u32)nx >> 1, pair_z = (olc_u32)ny * pair_y;
+    olc_u32 pair = (olc_u32)z0 * pair_z + (olc_u32)y * pair_y + ((olc_u32)x >> 1);
     unsigned short* o = out + ((size_t)z0 * ny + y) * nx + x;
     const int last = min(tz, nz - z0);
     // lanes past the grid compute (inside the box), but store nothing
@@ -269,10 +271,10 @@ __device__ __forceinline__ void t16_tile4(const unsigned short* tile, unsigned s
                 const int yy = y + m;
                 if (yy == 0 || yy == ny - 1 || z == 0 || z == nz - 1) v = b4;
             }
-            if (m < rows) store4w_at<ST, EN>(o + (size_t)m * nx, v, vi + (olc_u32)m * (olc_u32)nx, key, k);
+            if (m < rows) store4w_at<ST, EN>(o + (size_t)m * nx, v, pair + (olc_u32)m * pair_y, key, k);
         }
         o += (size_t)nx * ny;
-        vi += sz;
+        pair += pair_z;
     };
 #pragma unroll 1
     for (int lz = 1; lz <= last; lz += 2) {

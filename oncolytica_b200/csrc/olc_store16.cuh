@@ -230,12 +230,12 @@ __device__ __forceinline__ float4 load4w(const unsigned short* p, const EncConst
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// Four working values stored at voxel index vi (a multiple of 4).
+// Four working values stored; `pair` is half the first one's voxel index (a multiple of 4).
 template <int ST, int EN>
-__device__ __forceinline__ void store4w_at(unsigned short* p, const float4& v, olc_u32 vi, olc_u32 key,
+__device__ __forceinline__ void store4w_at(unsigned short* p, const float4& v, olc_u32 pair, olc_u32 key,
                                            const EncConst& k) {
-    const olc_u32 r0 = IsSR<ST>::value ? olc_sr_pair(vi >> 1, key) : 0u;
-    const olc_u32 r1 = IsSR<ST>::value ? olc_sr_pair((vi >> 1) + 1, key) : 0u;
+    const olc_u32 r0 = IsSR<ST>::value ? olc_sr_pair(pair, key) : 0u;
+    const olc_u32 r1 = IsSR<ST>::value ? olc_sr_pair(pair + 1, key) : 0u;
     *reinterpret_cast<uint2*>(p) = make_uint2(Codec<ST, EN>::pack(v.x, v.y, k, IsSR<ST>::value, r0),
                                               Codec<ST, EN>::pack(v.z, v.w, k, IsSR<ST>::value, r1));
 }

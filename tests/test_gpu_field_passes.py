@@ -148,3 +148,57 @@ def test_three_offset_substeps_bit_exact(cuda, olc, dims, storage):
     torch.cuda.synchronize()
     np.testing.assert_array_equal(fd.cpu().numpy().view(np.uint16).reshape(f.shape), bits)
     np.testing.assert_array_equal(cd.cpu().numpy().reshape(f.shape), comp)
+
+
+def _fmix32(h):
+    h ^= h >> 16
+    h = h * 0x85EBCA6B & 0xFFFFFFFF
+    h ^= h >> 13
+    h = h * 0xC2B2AE35 & 0xFFFFFFFF
+    return h ^ h >> 16
+
+
+def _fmix32_inverse(h):
+    h ^= h >> 16
+    h = h * pow(0xC2B2AE35, -1, 1 << 32) & 0xFFFFFFFF
+    h ^= h >> 13 ^ h >> 26
+    h = h * pow(0x85EBCA6B, -1, 1 << 32) & 0xFFFFFFFF
+    return h ^ h >> 16
+
+
+@pytest.mark.parametrize("storage", [3, 4])
+def test_three_offset_rounding_beyond_32_bit_voxel_indices(cuda, olc, storage):
+    """The planes of a field from voxel 2^32 on, against the oracle on those planes
+    alone.  Their pair indices carry bit 31; (p ^ 2^31) ^ key = p ^ (key ^ 2^31), so
+    the oracle takes the step whose key is that one."""
+    import torch
+
+    if torch.cuda.mem_get_info()[0] < 45 << 30:
+        pytest.skip("needs 36 GB of device memory")
+    nx, ny, k = 8, 32768, 9
+    nz = (1 << 32) // (nx * ny) + k
+    step, other = next((s, w >> 8) for s in range(1 << 16)
+                       for w in [_fmix32_inverse(_fmix32(s << 8) ^ 1 << 31)] if w & 0xFF == 0)
+    assert _fmix32(other << 8) == _fmix32(step << 8) ^ 1 << 31
+    b, dt = np.float32(0.7), 0.15
+    rng = np.random.default_rng(storage)
+    f = (b * rng.random((k, ny, nx))).astype(np.float32)
+    bits = oracle.to_bits16(f, storage, 2, b)
+    ref, _ = oracle.diffuse16(bits, None, np.zeros_like(f), 1.0, dt, 1.0, 0.05, float(b), 1, storage, step=other,
+                              field=0, encoding=2)
+    fd = torch.zeros((nz, ny, nx), dtype=torch.int16, device=cuda)
+    fd[-k:] = torch.from_numpy(bits.view(np.int16).reshape(k, ny, nx).copy()).to(cuda)
+    tmp = torch.zeros_like(fd)
+    cd = torch.zeros((nz, ny, nx), dtype=torch.float32, device=cuda)
+    spec = _lib.OlcDiffusion(diffusion=1.0, decay=0.05, boundary=float(b), substeps=1, has_sink=0, storage=storage,
+                             encoding=2)
+    dims_c = (C.c_int32 * 3)(nx, ny, nz)
+    _lib.check(olc.olc_stage_diffuse16(C.c_void_p(fd.data_ptr()), C.c_void_p(tmp.data_ptr()), None,
+                                       C.c_void_p(cd.data_ptr()), C.byref(dims_c), 1.0, dt, C.byref(spec), step, 0,
+                                       None))
+    got = fd[-k:].cpu().numpy().view(np.uint16)
+    del fd, tmp, cd
+    torch.cuda.empty_cache()
+    # the first plane is a face of the oracle's field alone, which its reaction leaves as it
+    # is (FP16: coding a decoded element again changes some), and the second one's neighbour
+    np.testing.assert_array_equal(got[2:], np.asarray(ref).reshape(k, ny, nx)[2:])
