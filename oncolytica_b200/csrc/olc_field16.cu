@@ -438,7 +438,7 @@ bool make_field_maps16(FieldMaps16* m, void* a, void* b, const int dims[3], int 
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const long long columns = (long long)((dims[0] + TX - 1) / TX) * ((dims[1] + TYR - 1) / TYR);
-        m->tz = 4;
+        m->tz = dims[2] > 4 * 65535 ? 8 : 4;  // at most 65,535 tiles along z
         while (m->tz > 1 && columns * ((dims[2] + m->tz - 1) / m->tz) < 12LL * sms) m->tz /= 2;
     }
     const cuuint32_t box[3] = {WX, WY, (cuuint32_t)(m->tz + 2)};

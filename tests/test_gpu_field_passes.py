@@ -202,3 +202,9 @@ def test_three_offset_rounding_beyond_32_bit_voxel_indices(cuda, olc, storage):
     # the first plane is a face of the oracle's field alone, which its reaction leaves as it
     # is (FP16: coding a decoded element again changes some), and the second one's neighbour
     np.testing.assert_array_equal(got[2:], np.asarray(ref).reshape(k, ny, nx)[2:])
+
+
+@pytest.mark.parametrize("nz", [262140, 262141, 300001])
+def test_three_offset_fields_of_many_planes(cuda, olc, nz):
+    """More planes than 65,535 tiles of four hold."""
+    test_three_offset_substeps_bit_exact(cuda, olc, (8, 3, nz), 3)
