@@ -337,6 +337,7 @@ bool make_march_plan(const int dims[3], float bval, int planes, MarchPlan* p, cu
             c.w = w;
             c.gx = (dims[1] - 2 + TYM - 3) / (TYM - 2);
             c.gy = (dims[0] + TX - 1) / TX;
+            if (c.gy > 65535) continue;  // the grid's limit; single passes have the columns in grid x
             const int nz = dims[2] - 2;  // interior planes
             const int resident = slots_sm * (16 / w);
             const int chunks = std::max(1, std::min(resident / (c.gx * c.gy), nz / 2));

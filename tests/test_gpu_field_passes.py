@@ -208,3 +208,29 @@ def test_three_offset_rounding_beyond_32_bit_voxel_indices(cuda, olc, storage):
 def test_three_offset_fields_of_many_planes(cuda, olc, nz):
     """More planes than 65,535 tiles of four hold."""
     test_three_offset_substeps_bit_exact(cuda, olc, (8, 3, nz), 3)
+
+
+@pytest.mark.parametrize("nx,ny", [(8388484, 16), (4194244, 32)])
+def test_rows_of_more_than_65535_tiles(cuda, olc, nx, ny):
+    """Rows of more columns of tiles than a grid has along y: the default passes
+    against single ones (another tile), on the device."""
+    import torch
+
+    if torch.cuda.mem_get_info()[0] < 30 << 30:
+        pytest.skip("needs 22 GB of device memory")
+    dims, dt = (nx, ny, 8), 0.3
+    g = torch.Generator(device=cuda).manual_seed(nx)
+    f = torch.rand(dims[::-1], generator=g, device=cuda)
+    spec = _lib.OlcDiffusion(diffusion=1.0, decay=0.03, boundary=0.6, substeps=2, has_sink=0)
+    dims_c = (C.c_int32 * 3)(*dims)
+    out = []
+    for tuning in (_lib.OlcTuning(8, 16, 0, 16, 0, 0, 0), None):
+        fd, tmp = f.clone(), torch.zeros_like(f)
+        _lib.check(olc.olc_stage_diffuse_tuned(C.c_void_p(fd.data_ptr()), C.c_void_p(tmp.data_ptr()), None,
+                                               C.byref(dims_c), 1.0, dt, C.byref(spec),
+                                               C.byref(tuning) if tuning is not None else None, None))
+        out.append(fd)
+    same = torch.equal(*out)
+    del f, fd, tmp, out
+    torch.cuda.empty_cache()
+    assert same
