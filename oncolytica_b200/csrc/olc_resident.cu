@@ -468,9 +468,9 @@ bool make_resident_plan(const int dims[3], bool groups, int sms, ResidentPlan* b
     const int nx = dims[0], ny = dims[1], nz = dims[2];
     const int G = (nx + 3) / 4;
     double best_cost = 1e30;
-    for (int By = 1; By <= ny; ++By) {
+    // at most one tile per SM along y, and 512 groups in a tile's plane
+    for (int By = (ny + sms - 1) / sms; By <= std::min(ny, 512 / G); ++By) {
         const int ty = (ny + By - 1) / By;
-        if (ty > sms) continue;
         const int tz_max = sms / ty;
         const int Bz = (nz + tz_max - 1) / tz_max;
         const int tz = (nz + Bz - 1) / Bz;
