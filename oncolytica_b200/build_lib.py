@@ -24,10 +24,12 @@ INCLUDE = os.path.join(REPO, "include")
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 
-SOURCES = ["olc_grid.cu", "olc_field.cu", "olc_march.cu", "olc_resident.cu", "olc_field16.cu", "olc_contact.cu", "olc_reduce.cu", "olc_batch.cu", "olc_sim.cu",
-           "olc_noalloc.cu", "olc_pool.cu", "olc_metrics.cu", "olc_selftest.cu"]
+SOURCES = ["olc_grid.cu", "olc_field.cu", "olc_march.cu", "olc_resident.cu", "olc_resident_bf16.cu",
+           "olc_resident_f16.cu", "olc_resident_bf16_sr.cu", "olc_resident_f16_sr.cu", "olc_field16.cu",
+           "olc_contact.cu", "olc_reduce.cu", "olc_batch.cu", "olc_sim.cu", "olc_noalloc.cu", "olc_pool.cu",
+           "olc_metrics.cu", "olc_selftest.cu"]
 HEADERS = ["olc_device.cuh", "olc_rule_rt.cuh", "olc_internal.h", "olc_store16.cuh", "olc_arena.h", "olc_stencil.cuh",
-           "olc_contact.cuh"]
+           "olc_contact.cuh", "olc_resident.cuh", "olc_resident16.cuh"]
 
 # -fmad=false keeps a*b+c as two roundings everywhere, so the CPU oracle
 # (compiled with -ffp-contract=off) reproduces every floating-point stage.
