@@ -392,6 +392,7 @@ bool make_field_maps(FieldMaps* m, float* a, float* b, const int dims[3], float 
     m->VY = tile_y;
     m->VZ = tile_z;
     m->passes = tile_y != 8 || tile_z != 8 || pair_threads > 0 || keep_pct > 0;
+    m->asked = pair_threads > 0;
     const cuuint32_t boxv[3] = {72, (cuuint32_t)(tile_y + 2), (cuuint32_t)(tile_z + 2)};
     if (!encode_map(&m->vec[0], a, dims, boxv) || !encode_map(&m->vec[1], b, dims, boxv)) return false;
     m->ok = true;
@@ -456,7 +457,7 @@ void launch_pins(float* f, const Pins* pins, cudaStream_t s) {
 // S substeps, one launch each; every other substep walks its tiles in reverse
 // order, so it starts on the tiles the previous one wrote last (still in L2).
 float* run_substeps_tma(float* a, float* b, const FieldMaps& m, int a_index, const FieldStep& fs, olc_u32* status,
-                        cudaStream_t s, const Pins* pins) {
+                        cudaStream_t s, const Pins* pins, bool in_place) {
     float* bufs[2];
     bufs[a_index] = a;
     bufs[1 - a_index] = b;
@@ -471,8 +472,14 @@ float* run_substeps_tma(float* a, float* b, const FieldMaps& m, int a_index, con
     }
     if (m.march.lx && !(pins && pins->n)) {
         // two substeps per launch (pinned voxels are re-pinned after every
-        // substep, so fields with pins take single passes)
-        for (; i + 1 < fs.substeps; i += 2) {
+        // substep, so fields with pins take single passes).  An odd number of passes
+        // leaves the result in the other buffer: where that means a copy, one pair is
+        // left to two single passes, unless pairs were asked for (256^3, 2 and 6
+        // substeps: 51.7 and 116.9 us with the copy, 42.1 and 112.4 without).  Rows
+        // of fewer than 32 voxels keep the copy (16 x 400 x 400, 2: 23 and 31).
+        const int left = fs.substeps - i, passes = left / 2 + (left & 1);
+        const bool copied = in_place && fs.dims[0] >= 32 && ((passes & 1) != 0) == (bufs[cur] == a);
+        for (int pairs = left / 2 - (copied && !m.asked ? 1 : 0); pairs > 0; --pairs, i += 2) {
             launch_march(m.march, m.march_map[cur], bufs[1 - cur], fs, status, (i >> 1) & 1, s);
             cur = 1 - cur;
         }

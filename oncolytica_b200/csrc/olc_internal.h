@@ -157,6 +157,7 @@ struct FieldMaps {
     CUtensorMap march_map[2];
     int keep = 0;  // planes [0, keep) kept L2-resident across substeps by eviction hints (0: none)
     bool passes = false;  // the caller's tuning names a shape of the passes: no other kernel instead of them
+    bool asked = false;   // the caller's tuning asks for two substeps per pass
 };
 // The TMA tensor maps of a FP32 field's two buffers for the (tile_y, tile_z)
 // tile; false when the tile is not compiled in or the field cannot be mapped
@@ -167,9 +168,10 @@ bool pair_threads_known(int nt);
 // Kernel launches of run_substeps_tma for one field step.
 int substep_launches(const FieldMaps& m, const FieldStep& fs, const Pins* pins);
 bool stencil_tile_known(int tile_y, int tile_z);
-// Runs fs.substeps substeps starting from a (buffer index a_index of m).
+// Runs fs.substeps substeps starting from a (buffer index a_index of m).  in_place:
+// the caller copies the result to a if it is in b.
 float* run_substeps_tma(float* a, float* b, const FieldMaps& m, int a_index, const FieldStep& fs, olc_u32* status,
-                        cudaStream_t s, const Pins* pins = nullptr);
+                        cudaStream_t s, const Pins* pins = nullptr, bool in_place = false);
 // All remaining substeps of a small field in one cooperative launch
 // (olc_resident.cu), after RESIDENT_LEAD ordinary ones.
 constexpr int RESIDENT_LEAD = 2;

@@ -2489,7 +2489,7 @@ static int stage_diffuse(float* f, float* tmp, float* sink, const int32_t dims[3
     if (status && make_field_maps(&maps, f, tmp, dims, spec->boundary, t->stencil_tile_y, t->stencil_tile_z, t->stencil_pair_threads,
                                   t->stencil_pair_planes, t->stencil_l2_keep_pct)) {
         launch_sink(f, spec->has_sink ? sink : nullptr, fs, st);
-        res = run_substeps_tma(f, tmp, maps, 0, fs, status, st);
+        res = run_substeps_tma(f, tmp, maps, 0, fs, status, st, nullptr, true);
     } else {
         res = run_field_step(f, tmp, spec->has_sink ? sink : nullptr, fs, status, st);
     }

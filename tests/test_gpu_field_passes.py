@@ -84,6 +84,27 @@ def test_two_substeps_per_pass_leave_negative_boundaries_to_single_passes(cuda, 
     _diffuse(cuda, olc, (64, 40, 20), 4, boundary=-0.25, tuning=_lib.OlcTuning(8, 8, 0, 16, 256, 0, 0))
 
 
+@pytest.mark.parametrize("substeps", [1, 2, 3, 4, 5, 6])
+def test_stage_of_a_large_field_ends_in_its_own_buffer(cuda, olc, substeps):
+    """A stage call whose passes would be odd in number takes one pair singly, so that
+    nothing is copied back: the other buffer holds the field before the last pass."""
+    import torch
+
+    dims, dt = (256, 256, 40), 0.15 * substeps
+    rng = np.random.default_rng(substeps)
+    f = rng.random(dims[::-1], dtype=np.float32)
+    ref = oracle.diffuse(f, None, dx=1.0, dt=dt, D=1.0, decay=0.03, boundary=0.6, substeps=substeps)
+    fd = torch.from_numpy(f.copy()).to(cuda)
+    tmp = torch.zeros_like(fd)
+    spec = _lib.OlcDiffusion(diffusion=1.0, decay=0.03, boundary=0.6, substeps=substeps)
+    dims_c = (C.c_int32 * 3)(*dims)
+    _lib.check(olc.olc_stage_diffuse(C.c_void_p(fd.data_ptr()), C.c_void_p(tmp.data_ptr()), None, C.byref(dims_c), 1.0,
+                                     dt, C.byref(spec), None))
+    np.testing.assert_array_equal(fd.cpu().numpy(), ref)
+    # one substep is one pass, whose result only a copy brings back
+    assert torch.equal(fd, tmp) == (substeps == 1)
+
+
 def test_large_field_takes_two_substeps_per_pass_by_itself(cuda, olc):
     _diffuse(cuda, olc, (256, 130, 140), 7, boundary=0.5)
 
