@@ -187,8 +187,19 @@ float* run_resident(float* in, float* other, const FieldStep& fs, int substeps, 
     return (substeps & 1) ? other : in;
 }
 
+// A 16-bit substep is shorter in passes and longer here than an FP32 one.  From a
+// million voxels on, where they fill the passes' tiles (at least four fifths), the
+// launch's fixed cost, about 10 us, is made up only at 10 substeps.  us in passes and
+// here, 6, 8 and 10 substeps: 128^3 30.2 and 33.2, 37.5 and 38.2, 48.5 and 45.4;
+// 256 x 64 x 64 24.8 and 29.0, 32.1 and 33.1, 38.3 and 37.2.  Else 6 are enough: 96^3
+// 24.9 and 22.9, 64^3 24.7 and 18.8, 64 x 24 x 900 (tiles three quarters full) 28.1
+// and 27.9.
 bool resident_fits16(const FieldStep& fs) {
-    return fs.encoding != OLC_ENC_OFFSET3 && resident_fits(fs);
+    auto tiles = [&](int axis, int size) { return (long long)((fs.dims[axis] + size - 1) / size) * size; };
+    const long long voxels = (long long)fs.dims[0] * fs.dims[1] * fs.dims[2];
+    const bool late = voxels >= 1000000 &&
+                      5 * voxels >= 4 * tiles(0, BATCH_T16_TX) * tiles(1, BATCH_T16_TY) * tiles(2, BATCH_T16_TZ);
+    return fs.encoding != OLC_ENC_OFFSET3 && fs.substeps >= (late ? 10 : 0) && resident_fits(fs);
 }
 
 // olc_resident16.cuh, a source file per storage type
