@@ -159,11 +159,13 @@ typedef struct {
     int32_t stencil_pair_threads; /* 128, 256, 512 or 1024 (one kernel serves all): two FP32
                                      substeps per pass (temporal blocking) where the field
                                      allows it (x extent a multiple of 4, at least 16 rows and
-                                     8 planes, boundary >= 0).  0 = the library's choice for
-                                     the field's size, or one substep per pass when a tile
-                                     other than (8, 8) or a kept slab is asked for */
-    int32_t stencil_pair_planes;  /* planes per CTA of the two-substep pass; 0 = as few
-                                     as keep the whole grid resident in one wave */
+                                     8 planes, boundary >= 0; else as 0).  0 = the library's
+                                     choice for the field's size, or one substep per pass when
+                                     a tile other than (8, 8), a kept slab or
+                                     stencil_pair_planes > 0 asks for that */
+    int32_t stencil_pair_planes;  /* planes per CTA of the two-substep pass, 0 = as few
+                                     as keep the whole grid resident in one wave; without
+                                     stencil_pair_threads, > 0 = one substep per pass */
     int32_t stencil_l2_keep_pct;  /* one-substep passes over an FP32 field read and write
                                      the first pct % of its planes with L2 evict_last
                                      and the rest with evict_first, so that slab of both

@@ -34,13 +34,13 @@ CONTACT_VARIANTS = (_lib.OLC_CONTACT_FLAT, _lib.OLC_CONTACT_NESTED)
 CONTACT_NAMES = {_lib.OLC_CONTACT_FLAT: "flat", _lib.OLC_CONTACT_NESTED: "nested"}
 BATCH_DEPTHS = (8, 16, 32)
 # (threads per CTA, planes per CTA) of the two-substeps-per-pass kernel, which serves every CTA size
-# alike; (0, 0) = the library's choice
-STENCIL_PAIRS = ((0, 0), (256, 0))
+# alike; (0, 0) = the library's choice, (0, 1) = one substep per pass
+STENCIL_PAIRS = ((0, 0), (0, 1), (256, 0))
 # share of an FP32 field's planes kept in L2 across one-substep passes (eviction hints)
 L2_KEEP = (0, 30, 45, 60)
 DEFAULT = {"stencil_tile": (8, 8), "contact_variant": _lib.OLC_CONTACT_FLAT, "batch_tile_depth": 16,
            "stencil_pair": (0, 0), "l2_keep_pct": 0}
-VERSION = 4  # cache entries of earlier tuners lack choices; they are measured again
+VERSION = 5  # cache entries of earlier tuners lack choices; they are measured again
 
 
 def pair_applies(threads: int, dims) -> bool:
@@ -55,7 +55,8 @@ def takes_pairs(tuning: dict, dims) -> bool:
     per pass under ``tuning``: asked for, or by the library's own choice, which the
     default shape leaves it for large fields (olc_march.cu march_pays)."""
     threads = tuple(tuning.get("stencil_pair", (0, 0)))[0]
-    own = tuple(tuning.get("stencil_tile", (8, 8))) == (8, 8) and not threads and not tuning.get("l2_keep_pct", 0)
+    own = (tuple(tuning.get("stencil_tile", (8, 8))) == (8, 8) and not any(tuning.get("stencil_pair", (0, 0)))
+           and not tuning.get("l2_keep_pct", 0))
     nx, ny, nz = (int(d) for d in dims)
     return (threads > 0 or (own and nx * ny * nz >= 1_000_000)) and pair_applies(256, dims)
 
@@ -162,7 +163,7 @@ def tune_engine(eng, steps: int = 4, cache: bool = True) -> dict:
             best["stencil_pair"] = min(times, key=times.get)
             measured["substep_pairs"] = {f"{a}/{b}": v for (a, b), v in times.items()}
             # the slab of planes kept in L2 from substep to substep
-            if best["stencil_pair"][0] == 0:
+            if best["stencil_pair"] == (0, 0):
                 times = {k: _measure(eng, sd, dict(best, l2_keep_pct=k), "ms_substeps", steps) for k in L2_KEEP}
                 best["l2_keep_pct"] = min(times, key=times.get)
                 measured["substep_l2_keep_pct"] = {str(k): v for k, v in times.items()}

@@ -368,9 +368,9 @@ class CudaBackend:
         """Kernel shapes and variants (olc_set_tuning): the FP32 stencil tile
         (rows, planes), the contact walk, the batched tile depth,
         ``stencil_pair`` = (threads per CTA, planes per CTA) of the
-        two-substeps-per-pass kernel ((0, 0): the library's choice), and the
-        share of an FP32 field's planes kept in L2 across substeps by
-        eviction hints (``l2_keep_pct``, 0: none)."""
+        two-substeps-per-pass kernel ((0, 0): the library's choice, (0, 1): one
+        substep per pass), and the share of an FP32 field's planes kept in L2
+        across substeps by eviction hints (``l2_keep_pct``, 0: none)."""
         t = _lib.OlcTuning(int(stencil_tile[0]), int(stencil_tile[1]), int(contact_variant), int(batch_tile_depth),
                            int(stencil_pair[0]), int(stencil_pair[1]), int(l2_keep_pct))
         self._check(self.lib.olc_set_tuning(self.handle, C.byref(t)))

@@ -391,16 +391,21 @@ bool make_field_maps(FieldMaps* m, float* a, float* b, const int dims[3], float 
     m->keep = (int)((long long)dims[2] * keep_pct / 100);
     m->VY = tile_y;
     m->VZ = tile_z;
-    m->passes = tile_y != 8 || tile_z != 8 || pair_threads > 0 || keep_pct > 0;
-    m->asked = pair_threads > 0;
+    m->single = pair_threads == 0 && pair_planes > 0;
+    m->passes = tile_y != 8 || tile_z != 8 || keep_pct > 0 || m->single;
+    m->asked = false;
     const cuuint32_t boxv[3] = {72, (cuuint32_t)(tile_y + 2), (cuuint32_t)(tile_z + 2)};
     if (!encode_map(&m->vec[0], a, dims, boxv) || !encode_map(&m->vec[1], b, dims, boxv)) return false;
     m->ok = true;
-    // two substeps per pass: when asked for, or, where no shape of the passes is, if that is faster
+    // two substeps per pass: when asked for, or, where single passes are not, if that is faster
     cuuint32_t box[3];
     if ((pair_threads > 0 || (!m->passes && march_pays(dims))) && make_march_plan(dims, bval, pair_planes, &m->march, box) &&
         (!encode_map(&m->march_map[0], a, dims, box) || !encode_map(&m->march_map[1], b, dims, box)))
         m->march.lx = 0;
+    // a pair the field does not allow leaves the choice to the library (256 x 12 x 256,
+    // 20 substeps: 93 us in single passes, 45 on chip)
+    m->asked = pair_threads > 0 && m->march.lx != 0;
+    m->passes = m->passes || m->asked;
     return true;
 }
 
@@ -523,10 +528,11 @@ void launch_substep(const float* in, float* out, const FieldStep& fs, cudaStream
                                                        fs.inv_decay, fs.bval);
 }
 
-float* run_substeps(float* a, float* b, const FieldStep& fs, olc_u32* status, cudaStream_t s, const Pins* pins) {
+float* run_substeps(float* a, float* b, const FieldStep& fs, olc_u32* status, cudaStream_t s, const Pins* pins,
+                    bool passes) {
     float* cur = a;
     float* nxt = b;
-    const bool resident = status && !(pins && pins->n) && resident_fits(fs);
+    const bool resident = status && !passes && !(pins && pins->n) && resident_fits(fs);
     for (int i = 0; i < fs.substeps; ++i) {
         if (resident && i == RESIDENT_LEAD)
             if (float* res = run_resident(cur, nxt, fs, fs.substeps - i, status, s)) return res;
@@ -540,9 +546,9 @@ float* run_substeps(float* a, float* b, const FieldStep& fs, olc_u32* status, cu
 }
 
 float* run_field_step(float* a, float* b, float* sink, const FieldStep& fs, olc_u32* status, cudaStream_t s,
-                      const Pins* pins) {
+                      const Pins* pins, bool passes) {
     launch_sink(a, sink, fs, s);
-    return run_substeps(a, b, fs, status, s, pins);
+    return run_substeps(a, b, fs, status, s, pins, passes);
 }
 
 }  // namespace olc

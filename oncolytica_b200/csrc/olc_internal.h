@@ -132,10 +132,10 @@ void launch_pins(float* f, const Pins* pins, cudaStream_t s);
 void launch_substep(const float* in, float* out, const FieldStep& fs, cudaStream_t s);
 // Runs sink + S substeps starting from a; returns the buffer holding the result.
 float* run_field_step(float* a, float* b, float* sink, const FieldStep& fs, olc_u32* status, cudaStream_t s,
-                      const Pins* pins = nullptr);
-// The S substeps alone.
+                      const Pins* pins = nullptr, bool passes = false);
+// The S substeps alone (passes: one launch each, whatever the field).
 float* run_substeps(float* a, float* b, const FieldStep& fs, olc_u32* status, cudaStream_t s,
-                    const Pins* pins = nullptr);
+                    const Pins* pins = nullptr, bool passes = false);
 // Two substeps per pass by warps marching along z (olc_march.cu).
 struct MarchPlan {
     int lx = 0;              // lanes per row, 0: the march does not apply
@@ -156,8 +156,9 @@ struct FieldMaps {
     MarchPlan march;     // two substeps per pass (lx 0: off)
     CUtensorMap march_map[2];
     int keep = 0;  // planes [0, keep) kept L2-resident across substeps by eviction hints (0: none)
-    bool passes = false;  // the caller's tuning names a shape of the passes: no other kernel instead of them
-    bool asked = false;   // the caller's tuning asks for two substeps per pass
+    bool single = false;  // the caller's tuning asks for one substep per pass, and for no shape of it
+    bool passes = false;  // it asks for passes or names a shape of them: no other kernel instead
+    bool asked = false;   // the caller's tuning asks for two substeps per pass, and the field allows it
 };
 // The TMA tensor maps of a FP32 field's two buffers for the (tile_y, tile_z)
 // tile; false when the tile is not compiled in or the field cannot be mapped

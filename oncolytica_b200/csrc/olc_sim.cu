@@ -385,13 +385,15 @@ int step_once(OlcSim* s, int collect, cudaStream_t st) {
         const Pins* pins = s->pins[f].n ? &s->pins[f] : nullptr;
         float* res = tma_path ? run_substeps_tma(a, b, s->fmaps[f], cur, s->fstep[f], s->counters + OLC_CTR_STATUS, st,
                                                  pins)
-                              : run_substeps(a, b, s->fstep[f], s->counters + OLC_CTR_STATUS, st, pins);
+                              : run_substeps(a, b, s->fstep[f], s->counters + OLC_CTR_STATUS, st, pins,
+                                             s->fmaps[f].single);
         s->field_cur[f] = (res == a) ? cur : 1 - cur;
         substeps += (uint32_t)s->fstep[f].substeps;
         launches += (uint64_t)(tma_path ? substep_launches(s->fmaps[f], s->fstep[f], pins)
                                         : (pins ? 2 * s->fstep[f].substeps
-                                                 : resident_fits(s->fstep[f]) ? RESIDENT_LEAD + 1
-                                                                              : s->fstep[f].substeps));
+                                                 : !s->fmaps[f].single && resident_fits(s->fstep[f])
+                                                     ? RESIDENT_LEAD + 1
+                                                     : s->fstep[f].substeps));
     }
     mark(s, 2, st);
     // 2. grid + compaction
@@ -2491,7 +2493,7 @@ static int stage_diffuse(float* f, float* tmp, float* sink, const int32_t dims[3
         launch_sink(f, spec->has_sink ? sink : nullptr, fs, st);
         res = run_substeps_tma(f, tmp, maps, 0, fs, status, st, nullptr, true);
     } else {
-        res = run_field_step(f, tmp, spec->has_sink ? sink : nullptr, fs, status, st);
+        res = run_field_step(f, tmp, spec->has_sink ? sink : nullptr, fs, status, st, nullptr, status && maps.single);
     }
     if (res != f) {
         const size_t bytes = (size_t)dims[0] * dims[1] * dims[2] * 4;

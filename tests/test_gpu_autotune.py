@@ -137,3 +137,39 @@ def test_batch_tile_depths_give_the_same_bits(cuda, tmp_path, monkeypatch):
     per = autotune.apply_batch(b, rec["depths"])
     assert len(per) == len(specs)
     assert autotune.tune_batch(lambda: W.build_batch(specs, states), steps=1)["cached"]
+
+
+def _launches_per_step(eng, **tuning):
+    be = eng._backend_impl
+    be.set_tuning(**tuning)
+    eng.run_steps(1)
+    be.set_profiling(True)
+    eng.run_steps(2)
+    prof = be.profile()
+    be.set_profiling(False)
+    return prof["kernel_launches"] / 2, prof["substep_launches"] / 2
+
+
+@pytest.mark.parametrize("dims", [(64, 64, 64), (50, 64, 64)])
+def test_one_substep_per_pass_can_be_asked_for(cuda, dims):
+    """(0, 1) takes a launch per substep, on rows that tensor maps describe and on
+    others, where the library's own choice takes three per field; same bits."""
+    spec = W.scaled(_spec(), field_dims=dims)
+    state = W.initial_state(spec)
+    ref = W.build_engine(spec, state)
+    own, substeps = _launches_per_step(ref)
+    eng = W.build_engine(spec, state)
+    single, _ = _launches_per_step(eng, stencil_pair=(0, 1))
+    fields = 2 if spec.S_drug else 1
+    assert single - own == substeps - 3 * fields
+    _same(eng._backend_impl.snapshot(), ref._backend_impl.snapshot(), "one substep per pass")
+
+
+def test_pairs_that_a_field_does_not_allow_leave_the_choice_to_the_library(cuda):
+    """Fewer than 16 rows: no two substeps per pass, and no single ones instead."""
+    spec = W.scaled(_spec(), field_dims=(64, 12, 64))
+    state = W.initial_state(spec)
+    ref = W.build_engine(spec, state)
+    eng = W.build_engine(spec, state)
+    assert _launches_per_step(eng, stencil_pair=(256, 0)) == _launches_per_step(ref)
+    _same(eng._backend_impl.snapshot(), ref._backend_impl.snapshot(), "pair on 12 rows")
