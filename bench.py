@@ -325,6 +325,7 @@ def run_b200(args) -> None:
         autotune.apply_engine(eng, tuning)
     eng.set_graphs(not args.no_graphs)
     be = eng._backend_impl
+    route = be.field_route("o2")  # the field with the most substeps
     dev = torch.device("cuda", local)
 
     def tuned(e):
@@ -458,21 +459,29 @@ def run_b200(args) -> None:
     sub_ms = prof["ms_substeps"] / max(1, prof["substep_launches"])  # per substep (a pair counts two)
     alg_bytes = 8 * nvox  # read 4 B + write 4 B per voxel and launch (FP32)
     t = tuning.get("tuning") or {}
-    paired = autotune.takes_pairs(t, spec.field_dims)
-    if paired:
+    subs = [S for S in (spec.S_o2, spec.S_drug) if S]
+    per_launch = 1
+    if route == "pairs":
         # two substeps per launch: the odd substep of each field is a single
         # pass, so a pair launch takes the fields' time less those singles,
         # timed at the best time per substep the tuner measured on a tile
         # shape, which takes one pass each (the default shape leaves the choice
         # to the library)
-        subs = [S for S in (spec.S_o2, spec.S_drug) if S]
         n_pairs = sum(S // 2 for S in subs)
         n_single = sum(S % 2 for S in subs)
         shapes = {k: v for k, v in tuning.get("measured_ms", {}).get("substeps", {}).items() if k != "8x8"}
         single_ms = min(shapes.values(), default=sub_ms * sum(subs)) / sum(subs)
         launch_ms = max(1e-6, (sub_ms * sum(subs) - n_single * single_ms) / max(1, n_pairs))
+        per_launch = 2
         kernel = "k_march2 (two 7-point FTCS substeps per pass, FP32, TMA plane ring)"
         traffic = read_traffic("k_march2", nvox)
+    elif route == "resident":
+        # a field's step is two single passes and one launch that keeps it on
+        # chip; the time is the launch's share by substeps
+        launch_ms = sub_ms * (sum(subs) - 2 * len(subs)) / len(subs)
+        per_launch = (sum(subs) - 2 * len(subs)) / len(subs)
+        kernel = "k_resident (a field's substeps but two in one launch, FP32, on chip)"
+        traffic = read_traffic("k_resident", nvox)
     else:
         launch_ms = sub_ms
         kernel = "k_substep_x4 (7-point FTCS, FP32, 4-wide rows, TMA tiles)"
@@ -492,7 +501,7 @@ def run_b200(args) -> None:
         "roofline": {"bound": "hbm", "kernel": kernel, "achieved": achieved,
                      "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
                      "peak_src": peaks["src"], "traffic": traffic, "alg_bytes_per_launch": alg_bytes,
-                     "launch_ms": launch_ms, "substeps_per_launch": 2 if paired else 1,
+                     "launch_ms": launch_ms, "substeps_per_launch": per_launch,
                      # one-substep-per-pass stream model (8 B per voxel-substep): above 1.0
                      # only when passes carry more than one substep
                      "per_substep_us": sub_ms * 1e3,

@@ -179,6 +179,13 @@ typedef struct {
  * waits for the device. */
 int olc_set_tuning(OlcSim* sim, const OlcTuning* tuning);
 int olc_get_tuning(const OlcSim* sim, OlcTuning* out);
+/* How a solo handle's bound field takes its substeps under the handle's tuning: a
+ * launch per substep, per two (an odd one singly), or the first two singly and the
+ * others in one launch that keeps the field on chip.  Every route gives the same bits. */
+#define OLC_ROUTE_PASSES   0
+#define OLC_ROUTE_PAIRS    1
+#define OLC_ROUTE_RESIDENT 2
+int olc_field_route(const OlcSim* sim, uint32_t field, int32_t* route);
 /* Batch handles: the batched FP32 substep tile depth of each member (n =
  * members; 0 = the handle's batch_tile_depth), so each grid size can take the
  * depth measured fastest for it. */

@@ -50,17 +50,6 @@ def pair_applies(threads: int, dims) -> bool:
     return threads == 0 or (nx % 4 == 0 and ny >= 16 and nz >= 8)
 
 
-def takes_pairs(tuning: dict, dims) -> bool:
-    """Whether FP32 fields of ``dims`` (with a boundary value >= +0) take two substeps
-    per pass under ``tuning``: asked for, or by the library's own choice, which the
-    default shape leaves it for large fields (olc_march.cu march_pays)."""
-    threads = tuple(tuning.get("stencil_pair", (0, 0)))[0]
-    own = (tuple(tuning.get("stencil_tile", (8, 8))) == (8, 8) and not any(tuning.get("stencil_pair", (0, 0)))
-           and not tuning.get("l2_keep_pct", 0))
-    nx, ny, nz = (int(d) for d in dims)
-    return (threads > 0 or (own and nx * ny * nz >= 1_000_000)) and pair_applies(256, dims)
-
-
 CACHE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_cache", "tuning.json")
 _lock = threading.Lock()
 
@@ -263,5 +252,5 @@ def summary(rec: dict) -> dict:
     return out
 
 
-__all__ = ["tune_engine", "tune_batch", "apply_engine", "apply_batch", "summary", "pair_applies", "takes_pairs",
-           "STENCIL_TILES", "STENCIL_PAIRS", "L2_KEEP", "CONTACT_VARIANTS", "BATCH_DEPTHS"]
+__all__ = ["tune_engine", "tune_batch", "apply_engine", "apply_batch", "summary", "pair_applies", "STENCIL_TILES",
+           "STENCIL_PAIRS", "L2_KEEP", "CONTACT_VARIANTS", "BATCH_DEPTHS"]

@@ -382,6 +382,14 @@ class CudaBackend:
                 "batch_tile_depth": t.batch_tile_depth,
                 "stencil_pair": (t.stencil_pair_threads, t.stencil_pair_planes), "l2_keep_pct": t.stencil_l2_keep_pct}
 
+    def field_route(self, name: str) -> str:
+        """How a diffusing field takes its substeps (olc_field_route): "passes" (a
+        launch each), "pairs" (two per launch) or "resident" (two passes, then the
+        others in one launch)."""
+        r = C.c_int32()
+        self._check(self.lib.olc_field_route(self.handle, list(self.layout.chem_fields).index(name), C.byref(r)))
+        return ("passes", "pairs", "resident")[r.value]
+
     def has_tma_fields(self) -> bool:
         """Whether a diffusing FP32 field takes the TMA substep (the tuned tile)."""
         eng = self.engine

@@ -468,7 +468,8 @@ float* run_substeps_tma(float* a, float* b, const FieldMaps& m, int a_index, con
     bufs[1 - a_index] = b;
     int cur = a_index;
     int i = 0;
-    if (!m.passes && !(pins && pins->n) && resident_fits(fs)) {
+    const int route = substep_route(m, fs, pins);
+    if (route == OLC_ROUTE_RESIDENT) {
         for (; i < RESIDENT_LEAD; ++i) {
             launch_single(m, cur, bufs[1 - cur], fs, status, i & 1, s);
             cur = 1 - cur;
@@ -497,11 +498,16 @@ float* run_substeps_tma(float* a, float* b, const FieldMaps& m, int a_index, con
     return bufs[cur];
 }
 
-int substep_launches(const FieldMaps& m, const FieldStep& fs, const Pins* pins) {
+int substep_route(const FieldMaps& m, const FieldStep& fs, const Pins* pins) {
+    if (pins && pins->n) return OLC_ROUTE_PASSES;
+    if (!(m.ok ? m.passes : m.single) && resident_fits(fs)) return OLC_ROUTE_RESIDENT;
+    return m.ok && m.march.lx ? OLC_ROUTE_PAIRS : OLC_ROUTE_PASSES;
+}
+
+int substep_launches(int route, const FieldStep& fs, const Pins* pins) {
     if (pins && pins->n) return 2 * fs.substeps;
-    if (!m.passes && resident_fits(fs)) return RESIDENT_LEAD + 1;
-    if (m.ok && m.march.lx) return fs.substeps / 2 + (fs.substeps & 1);
-    return fs.substeps;
+    if (route == OLC_ROUTE_RESIDENT) return RESIDENT_LEAD + 1;
+    return route == OLC_ROUTE_PAIRS ? fs.substeps / 2 + (fs.substeps & 1) : fs.substeps;
 }
 
 // Status word of the stateless stage entry points (bounded waits report here).

@@ -166,8 +166,10 @@ struct FieldMaps {
 bool make_field_maps(FieldMaps* m, float* a, float* b, const int dims[3], float bval, int tile_y = 8, int tile_z = 8,
                      int pair_threads = 0, int pair_planes = 0, int keep_pct = 0);
 bool pair_threads_known(int nt);
-// Kernel launches of run_substeps_tma for one field step.
-int substep_launches(const FieldMaps& m, const FieldStep& fs, const Pins* pins);
+// How run_substeps_tma (or run_substeps, where the maps are not ok) takes a field's
+// substeps (OLC_ROUTE_*), and the kernel launches of one field step so.
+int substep_route(const FieldMaps& m, const FieldStep& fs, const Pins* pins);
+int substep_launches(int route, const FieldStep& fs, const Pins* pins);
 bool stencil_tile_known(int tile_y, int tile_z);
 // Runs fs.substeps substeps starting from a (buffer index a_index of m).  in_place:
 // the caller copies the result to a if it is in b.

@@ -342,6 +342,13 @@ void mark(OlcSim* s, int k, cudaStream_t st) {
     cudaEventRecord(s->events[s->prof_step][k], st);
 }
 
+// OLC_ROUTE_* of a bound field.
+int field_route(const OlcSim* s, olc_u32 f) {
+    if (s->fstep[f].storage != OLC_FIELD_F32)
+        return resident_fits16(s->fstep[f]) ? OLC_ROUTE_RESIDENT : OLC_ROUTE_PASSES;
+    return substep_route(s->fmaps[f], s->fstep[f], &s->pins[f]);
+}
+
 int step_once(OlcSim* s, int collect, cudaStream_t st) {
     const olc_u32 cap = s->caps.max_agents;
     if (s->profiling) {
@@ -376,7 +383,7 @@ int step_once(OlcSim* s, int collect, cudaStream_t st) {
                                        s->counters + OLC_CTR_STATUS, s->counters + OLC_CTR_FIELD_STEP, 0u, (int)f, st);
             s->field_cur[f] = (res == s->field[cur][f]) ? cur : 1 - cur;
             substeps += (uint32_t)s->fstep[f].substeps;
-            launches += (uint64_t)(resident_fits16(s->fstep[f]) ? RESIDENT_LEAD + 1 : s->fstep[f].substeps);
+            launches += (uint64_t)substep_launches(field_route(s, f), s->fstep[f], nullptr);
             continue;
         }
         float* a = s->field[cur][f];
@@ -389,11 +396,7 @@ int step_once(OlcSim* s, int collect, cudaStream_t st) {
                                              s->fmaps[f].single);
         s->field_cur[f] = (res == a) ? cur : 1 - cur;
         substeps += (uint32_t)s->fstep[f].substeps;
-        launches += (uint64_t)(tma_path ? substep_launches(s->fmaps[f], s->fstep[f], pins)
-                                        : (pins ? 2 * s->fstep[f].substeps
-                                                 : !s->fmaps[f].single && resident_fits(s->fstep[f])
-                                                     ? RESIDENT_LEAD + 1
-                                                     : s->fstep[f].substeps));
+        launches += (uint64_t)substep_launches(field_route(s, f), s->fstep[f], pins);
     }
     mark(s, 2, st);
     // 2. grid + compaction
@@ -2743,6 +2746,15 @@ int olc_set_tuning(OlcSim* s, const OlcTuning* t) {
 int olc_get_tuning(const OlcSim* s, OlcTuning* out) {
     if (!s || !out) return fail(nullptr, OLC_ERR_ARG, "olc_get_tuning: null argument");
     *out = s->tuning;
+    return OLC_OK;
+}
+
+int olc_field_route(const OlcSim* s, uint32_t field, int32_t* route) {
+    if (!s || !route) return fail(nullptr, OLC_ERR_ARG, "olc_field_route: null argument");
+    if (s->n_sims) return fail(nullptr, OLC_ERR_STATE, "olc_field_route: not a solo handle");
+    if (field >= s->caps.n_fields || !s->field_bound[field] || s->fstep[field].substeps == 0)
+        return fail(nullptr, OLC_ERR_ARG, "olc_field_route: no such diffusing field");
+    *route = field_route(s, field);
     return OLC_OK;
 }
 

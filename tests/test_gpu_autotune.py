@@ -173,3 +173,24 @@ def test_pairs_that_a_field_does_not_allow_leave_the_choice_to_the_library(cuda)
     eng = W.build_engine(spec, state)
     assert _launches_per_step(eng, stencil_pair=(256, 0)) == _launches_per_step(ref)
     _same(eng._backend_impl.snapshot(), ref._backend_impl.snapshot(), "pair on 12 rows")
+
+
+@pytest.mark.parametrize("dims,tuning,route", [
+    ((64, 64, 64), {}, "resident"), ((50, 64, 64), {}, "resident"), ((64, 64, 64), {"stencil_pair": (0, 1)}, "passes"),
+    ((50, 64, 64), {"stencil_pair": (0, 1)}, "passes"), ((64, 64, 64), {"stencil_pair": (256, 0)}, "pairs"),
+    ((64, 64, 64), {"stencil_tile": (16, 8)}, "passes"), ((128, 128, 128), {}, "resident"),
+    ((160, 160, 160), {}, "pairs"), ((150, 160, 160), {}, "passes")])
+def test_the_route_of_a_field_is_the_librarys_to_say(cuda, dims, tuning, route):
+    """Small fields stay on chip, up to sizes beyond the least the pairs take; what
+    olc_field_route says is what the launches show."""
+    spec = W.scaled(_spec(), field_dims=dims)
+    eng = W.build_engine(spec)
+    got, substeps = _launches_per_step(eng, **tuning)
+    assert [eng._backend_impl.field_route(n) for n in ("o2", "drug")] == [route] * 2
+    ref = W.build_engine(W.scaled(spec, field_dims=(64, 64, 64)))
+    own, _ = _launches_per_step(ref)  # three per field
+    S = [spec.S_o2, spec.S_drug]
+    per = {"resident": 6, "pairs": sum(s // 2 + s % 2 for s in S), "passes": sum(S)}[route]
+    assert got - own == per - 6
+    with pytest.raises(_lib.OlcError):
+        _lib.check(eng._backend_impl.lib.olc_field_route(eng._backend_impl.handle, 7, None))
