@@ -666,6 +666,18 @@ int olc_sort_noalloc_status(uint32_t* status_out, void* stream);
  * reference. */
 int olc_selftest_bounded_waits(uint32_t limit, uint32_t out[3], void* stream);
 
+/* The same for the exchange of a field that stays on chip: launches one of a field's
+ * two tiles, whose wait for the other runs out after 1,000 polls, and records
+ * OLC_STATUS_TIMEOUT where the stage entry points do (olc_stage_status). */
+int olc_selftest_exchange_wait(void* stream);
+
+/* The status bits (OLC_STATUS_*) that stage calls on the current device have recorded
+ * since the last read, which clears them; waits for `stream`.  The field stages wait
+ * on the device, for copies and for one another's tiles, and a wait that runs out
+ * (OLC_STATUS_TIMEOUT) leaves a wrong field behind: the calls themselves return
+ * before their kernels have run.  (Sorts have a status word of their own.) */
+int olc_stage_status(uint32_t* bits, void* stream);
+
 /* Bin table from sorted keys: ranges_dev[2k] = first index of key k,
  * ranges_dev[2k+1] = one past the last (both 0 when empty); keys >= n_bins are
  * ignored.  Replaces VoxelTable.startIndex/count (template.wgsl:42-45). */

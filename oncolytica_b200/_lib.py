@@ -56,7 +56,8 @@ EXPORTS = (
     "olc_engine_metrics", "olc_get_step_state", "olc_set_step_state", "olc_set_mechanics",
     "olc_stage_contact_mech", "olc_stage_contact_motion", "olc_bind_tissue_pair", "olc_current_tissue", "olc_set_rule_iterations",
     "olc_set_pinned", "olc_stage_diffuse_pinned", "olc_sort_noalloc_status", "olc_sort_status_offset",
-    "olc_selftest_bounded_waits", "olc_set_tuning", "olc_get_tuning", "olc_field_route", "olc_set_batch_tile_depths",
+    "olc_selftest_bounded_waits", "olc_selftest_exchange_wait", "olc_stage_status", "olc_set_tuning", "olc_get_tuning",
+    "olc_field_route", "olc_set_batch_tile_depths",
     "olc_stage_diffuse_tuned", "olc_stage_contact_tuned", "olc_queue_readback", "olc_take_readback",
 )
 
@@ -428,6 +429,8 @@ _SIGS = {
     "olc_sort_noalloc_status": (C.c_int, [C.POINTER(C.c_uint32), _VP]),
     "olc_sort_status_offset": (C.c_size_t, []),
     "olc_selftest_bounded_waits": (C.c_int, [C.c_uint32, C.POINTER(C.c_uint32 * 3), _VP]),
+    "olc_selftest_exchange_wait": (C.c_int, [_VP]),
+    "olc_stage_status": (C.c_int, [C.POINTER(C.c_uint32), _VP]),
     "olc_set_tuning": (C.c_int, [_VP, C.POINTER(OlcTuning)]),
     "olc_field_route": (C.c_int, [_VP, C.c_uint32, C.POINTER(C.c_int32)]),
     "olc_get_tuning": (C.c_int, [_VP, C.POINTER(OlcTuning)]),

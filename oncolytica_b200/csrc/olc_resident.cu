@@ -45,6 +45,7 @@ struct ResidentF32 {
         if (left > 3) olc_st_relaxed(w + 3, q.w);
     }
     static constexpr olc_u32 PHASE = 0x80000000u;
+    static constexpr olc_u32 POLLS = OLC_SPIN_LIMIT;  // of one exchange; an argument cost 64^3 3 % of its time
     static __device__ __forceinline__ olc_u32 load_word(const void* f, olc_u32 v) {
         return olc_ld_relaxed(static_cast<const olc_u32*>(f) + v);
     }
@@ -230,3 +231,44 @@ void* run_resident16(void* in, void* other, const FieldStep& fs, int substeps, o
 }
 
 }  // namespace olc
+
+// A field of two tiles of which only the first is launched: its exchange with the
+// second waits for words that nobody publishes, gives up and reports it.
+namespace {
+constexpr int SELFTEST_DIMS[3] = {16, 8, 4};
+__device__ __align__(16) float g_selftest_field[2][16 * 8 * 4];
+}  // namespace
+
+namespace olc {
+namespace {
+struct ResidentSelftest : ResidentF32<true> {
+    static constexpr olc_u32 POLLS = 1000;
+};
+}  // namespace
+}  // namespace olc
+
+extern "C" int olc_selftest_exchange_wait(void* stream) {
+    using namespace olc;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    void* buf = nullptr;
+    olc_u32* status = stage_status_word();
+    cudaError_t e = cudaGetSymbolAddress(&buf, g_selftest_field);
+    if (e != cudaSuccess || !status) return cuda_status(cudaErrorSymbolNotFound, "olc_selftest_exchange_wait");
+    e = cudaMemsetAsync(buf, 0, sizeof(g_selftest_field), st);
+    if (e != cudaSuccess) return cuda_status(e, "olc_selftest_exchange_wait: clear");
+    FieldStep fs = {};
+    for (int i = 0; i < 3; ++i) fs.dims[i] = SELFTEST_DIMS[i];
+    fs.r = 0.1f;
+    fs.inv_decay = 1.0f;
+    ResidentPlan p;
+    p.By = p.Bz = p.runs = 4;
+    p.ty = 2;
+    p.tz = p.K = p.RI = p.L = 1;
+    p.NT = 256;
+    p.smem = (size_t)(p.By + 2) * 2 * (p.Bz + 2) * (SELFTEST_DIMS[0] / 4) * 16;
+    ResidentArgs a;
+    float* f = static_cast<float*>(buf);
+    fill_resident_args(&a, f, f + sizeof(g_selftest_field) / 8, fs, p, 3, status);
+    p.ty = 1;  // the launch's share of them
+    return cuda_status(launch_resident_t<1, 256, 1, false, ResidentSelftest>(a, p, st), "olc_selftest_exchange_wait");
+}

@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const ResidentArgs a) {
         // tiles still computing would wait behind them.
         auto wait_more = [&]() {
             if (gave_up) return false;
-            if (++spins <= OLC_SPIN_LIMIT) return true;
+            if (++spins <= E::POLLS) return true;
             atomicOr(a.status, OLC_ST_TIMEOUT);
             gave_up = true;
             return false;

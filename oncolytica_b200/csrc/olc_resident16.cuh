@@ -14,6 +14,7 @@ struct Resident16 {
     typedef uint2 Raw;
     static constexpr bool GROUPS = true;
     static constexpr olc_u32 PHASE = 0x80008000u;
+    static constexpr olc_u32 POLLS = OLC_SPIN_LIMIT;
     static __device__ __forceinline__ Raw load(const void* f, olc_u32 v, int, olc_u32) {
         uint2 q;
         asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];"

@@ -2473,6 +2473,16 @@ int olc_stage_bin_ranges(const uint32_t* keys, uint32_t n, uint32_t n_bins, uint
     return cuda_status(cudaGetLastError(), "olc_stage_bin_ranges");
 }
 
+int olc_stage_status(uint32_t* bits, void* stream) {
+    if (!bits) return fail(nullptr, OLC_ERR_ARG, "olc_stage_status: null argument");
+    olc_u32* word = stage_status_word();
+    if (!word) return cuda_status(cudaGetLastError(), "olc_stage_status: device word");
+    cudaStream_t st = as_stream(stream);
+    cudaMemcpyAsync(bits, word, 4, cudaMemcpyDeviceToHost, st);
+    cudaMemsetAsync(word, 0, 4, st);
+    return cuda_status(cudaStreamSynchronize(st), "olc_stage_status");
+}
+
 static int stage_diffuse(float* f, float* tmp, float* sink, const int32_t dims[3], float dx, float dt,
                          const OlcDiffusion* spec, const OlcTuning* t, void* stream, const char* who) {
     if (!f || !tmp || !dims || !spec) return fail(nullptr, OLC_ERR_ARG, std::string(who) + ": null argument");

@@ -122,3 +122,25 @@ def test_status_policies_warn_and_ignore(cuda):
     eng = _overflowing_engine("ignore")
     eng.run_step(collect_metrics=True)
     assert eng._backend_impl.counters()["status"] & _lib.OLC_STATUS_CAPACITY
+
+
+def test_an_exchange_that_nobody_answers_gives_up_and_is_reported(cuda, olc):
+    """One of the two tiles of a field that stays on chip runs alone: it gives up after
+    its polls, the stage status says so once, and the same route still runs clean."""
+    import torch
+
+    bits = C.c_uint32(7)
+    _lib.check(olc.olc_stage_status(C.byref(bits), None))  # whatever earlier stage calls left
+    _lib.check(olc.olc_selftest_exchange_wait(None))
+    _lib.check(olc.olc_stage_status(C.byref(bits), None))
+    assert bits.value == _lib.OLC_STATUS_TIMEOUT
+    f = torch.full((64, 64, 64), 0.5, device=cuda)
+    tmp = torch.zeros_like(f)
+    dims = (C.c_int32 * 3)(64, 64, 64)
+    spec = _lib.OlcDiffusion(diffusion=1.0, boundary=0.5, substeps=12)
+    _lib.check(olc.olc_stage_diffuse(C.c_void_p(f.data_ptr()), C.c_void_p(tmp.data_ptr()), None, C.byref(dims), 1.0, 1.2,
+                                     C.byref(spec), None))
+    _lib.check(olc.olc_stage_status(C.byref(bits), None))
+    assert bits.value == 0
+    assert torch.all(f == 0.5)
+    assert olc.olc_stage_status(None, None) == _lib.OLC_ERR_ARG
