@@ -309,16 +309,21 @@ __global__ void __launch_bounds__(CW_THREADS) k_contact_warp(const float4* __res
 // The flat walk (OLC_CONTACT_FLAT) is a warp per eight agents up to CW_MAX rows of
 // capacity, a thread per agent above, where it fills the SMs: us with a warp and with
 // a thread at 10,000 rows 13 and 26, 40,000 25 and 35 (22 and 21 if sparse, 35 and
-// 51 if dense), 80,000 38 and 39, 120,000 52 and 45, 1 M 374 and 274.  The nested
+// 51 if dense), 80,000 38 and 39, 120,000 52 and 45, 1 M 374 and 274.  A warp spends
+// about 250 instructions on every occupied bin, which sparse agents do not share, so a
+// known number of rows from CW_SPARSE up with more than two bins of the grid per row
+// gets threads (49,000 agents, 0.2 and 0.7 per bin: 23 and 10, 23 and 13).  The nested
 // loops of k_contact are the other choice (OlcTuning.contact_variant); all give the
 // same bits.
-constexpr olc_u32 CW_MAX = 49152;
+constexpr olc_u32 CW_MAX = 49152, CW_SPARSE = 20000;
 void launch_contact(const float4* posr, const olc_u32* ranges, const olc_u32* n_dev, olc_u32 n_host,
                     olc_u32 n_cap, const ContactDev& c, float* x, float* y, float* z, cudaStream_t s, int variant,
                     olc_u32 n_table) {
     if (variant != OLC_CONTACT_NESTED) {
         const uint2* rg = reinterpret_cast<const uint2*>(ranges);
-        if (n_cap <= CW_MAX) {
+        const long long bins = (long long)c.tdims[0] * c.tdims[1] * c.tdims[2];
+        const bool sparse = !n_dev && n_host >= CW_SPARSE && bins > 2LL * n_host;
+        if (n_cap <= CW_MAX && !sparse) {
             const olc_u32 blocks = n_cap == 0 ? 1 : (n_cap + CW_BLOCK - 1) / CW_BLOCK;
             k_contact_warp<<<blocks, CW_THREADS, 0, s>>>(posr, rg, n_dev, n_host, c, x, y, z);
             return;

@@ -101,3 +101,41 @@ def test_contact_lists_that_fill_in_mid_bin(cuda, olc, agents, per_bin):
         _lib.check(olc.olc_stage_contact(ptr[0], ptr[1], agents, C.byref(g), C.byref(spec), 0.1, *ptr[2:], None))
         torch.cuda.synchronize()
         np.testing.assert_array_equal(np.stack([t.cpu().numpy() for t in xyz], axis=1), ref)
+
+
+@pytest.mark.parametrize("per_bin", [0.1, 0.4, 0.6, 2.4])
+@pytest.mark.parametrize("agents", [19999, 20000, 24640, 30001, 49152])
+def test_sparse_agents_get_a_thread_each(cuda, olc, agents, per_bin):
+    """Sizes on either side of the least where sparse agents get a thread each, at grids
+    of more and fewer bins than that takes: at faces, with dead agents, and with pairs
+    that touch."""
+    import torch
+
+    rng = np.random.default_rng(agents + int(100 * per_bin))
+    vs = 10.0
+    d = max(4, 2 * int(round((agents / per_bin) ** (1 / 3) / 2)))
+    dims = (min(d, 120),) * 3
+    top = np.array(dims) * vs
+    pos = rng.uniform(0.0, 1.0, (agents, 3)) * top
+    pairs = rng.random(agents) < 0.3  # close to another one
+    pos[pairs] = pos[rng.integers(0, agents, int(pairs.sum()))] + rng.uniform(-6, 6, (int(pairs.sum()), 3))
+    pos = np.clip(pos, 0.0, top - 0.01).astype(np.float32)
+    ks, perm = oracle.sort_pairs(oracle.keys(pos, dims, vs))
+    ranges = oracle.bin_ranges(ks, oracle.tissue_key(*dims)).reshape(-1, 2).copy()
+    posr = np.concatenate([pos[perm], rng.uniform(4.0, 6.0, (agents, 1))], axis=1).astype(np.float32)
+    posr[rng.random(agents) < 0.1, 3] = -1.0
+    lo, hi = (0.1, 0.1, 0.1), tuple(float(t) - 0.1 for t in top)
+    ref = oracle.contact(posr, ranges.reshape(-1), dims, vs, 1.0, 10.0, 1.0, 0.1, lo, hi)
+    pr = torch.from_numpy(posr).to(cuda)
+    rg = torch.from_numpy(ranges.astype(np.uint32).view(np.int32).copy()).to(cuda)
+    xyz = [torch.from_numpy(np.ascontiguousarray(posr[:, a])).to(cuda) for a in range(3)]
+    g = _lib.OlcGeom()
+    g.tissue_dims[:] = dims
+    g.tissue_voxel_size = vs
+    g.chem_voxel_size = 1.0
+    g.domain_hi[:] = tuple(float(t) for t in top)
+    spec = _lib.OlcContact(enabled=1, radius_field=-1, stiffness=1.0, mobility=10.0, max_disp=1.0, margin=0.1)
+    ptr = [C.c_void_p(t.data_ptr()) for t in (pr, rg, *xyz)]
+    _lib.check(olc.olc_stage_contact(ptr[0], ptr[1], agents, C.byref(g), C.byref(spec), 0.1, *ptr[2:], None))
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(np.stack([t.cpu().numpy() for t in xyz], axis=1), ref)
