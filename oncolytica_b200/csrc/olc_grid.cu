@@ -98,8 +98,12 @@ __global__ void __launch_bounds__(256) k_keys(const float* __restrict__ x, const
 // upper digits, alike over thousands of keys, cost an atomic per thread and not one
 // per key, and the lowest, spread over the bins, meet few conflicts.  4 M keys, 4
 // passes: 61 us with a vote per key and pass and eight small blocks per SM, 14 so.
-constexpr int HIST_KEYS = 16, HIST_THREADS = 512;
-template <int PASSES>
+// Up to HIST_FEW keys a thread takes HIST_KEYS_FEW: with 16 the blocks are too few and
+// each thread's chain too long (80,000 keys in ten blocks 5.2 us, in forty 3.9; the
+// whole sort of 65,537 to 262,144 rows of 30 bits 2 us shorter).
+constexpr int HIST_KEYS = 16, HIST_KEYS_FEW = 4, HIST_THREADS = 512;
+constexpr olc_u32 HIST_FEW = 262144;
+template <int PASSES, int KEYS>
 __global__ void __launch_bounds__(HIST_THREADS) k_digit_hist(const olc_u32* __restrict__ keys, const olc_u32* n_dev,
                                                              olc_u32 n_host, olc_u32* __restrict__ hist) {
     __shared__ olc_u32 sh[PASSES][RADIX];
@@ -107,13 +111,13 @@ __global__ void __launch_bounds__(HIST_THREADS) k_digit_hist(const olc_u32* __re
     for (int i = threadIdx.x; i < PASSES * RADIX; i += HIST_THREADS) (&sh[0][0])[i] = 0u;
     __syncthreads();
     const bool wide = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0u;
-    for (olc_u64 at = ((olc_u64)blockIdx.x * HIST_THREADS + threadIdx.x) * HIST_KEYS; at < n;
-         at += (olc_u64)gridDim.x * HIST_THREADS * HIST_KEYS) {
-        olc_u32 k[HIST_KEYS];
-        const olc_u32 have = (olc_u32)min((olc_u64)HIST_KEYS, n - at);
-        if (wide && have == HIST_KEYS) {
+    for (olc_u64 at = ((olc_u64)blockIdx.x * HIST_THREADS + threadIdx.x) * KEYS; at < n;
+         at += (olc_u64)gridDim.x * HIST_THREADS * KEYS) {
+        olc_u32 k[KEYS];
+        const olc_u32 have = (olc_u32)min((olc_u64)KEYS, n - at);
+        if (wide && have == KEYS) {
 #pragma unroll
-            for (int j = 0; j < HIST_KEYS / 4; ++j) {
+            for (int j = 0; j < KEYS / 4; ++j) {
                 const uint4 v = reinterpret_cast<const uint4*>(keys + at)[j];
                 k[4 * j] = v.x;
                 k[4 * j + 1] = v.y;
@@ -122,13 +126,13 @@ __global__ void __launch_bounds__(HIST_THREADS) k_digit_hist(const olc_u32* __re
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < HIST_KEYS; ++j) k[j] = keys[at + min((olc_u32)j, have - 1)];
+            for (int j = 0; j < KEYS; ++j) k[j] = keys[at + min((olc_u32)j, have - 1)];
         }
 #pragma unroll
         for (int p = 0; p < PASSES; ++p) {
             olc_u32 run = 0, d = (k[0] >> (8 * p)) & 0xffu;
 #pragma unroll
-            for (int j = 0; j < HIST_KEYS; ++j) {
+            for (int j = 0; j < KEYS; ++j) {
                 const olc_u32 e = (k[j] >> (8 * p)) & 0xffu;
                 if (e != d) {
                     atomicAdd(&sh[p][d], run);
@@ -517,17 +521,26 @@ void launch_keys(const float* x, const float* y, const float* z, const unsigned 
                                   dead_ctr);
 }
 
-void launch_digit_hist(const olc_u32* keys, const olc_u32* n_dev, olc_u32 n_host, olc_u32 n_cap,
-                       olc_u32* hist, int passes, cudaStream_t s) {
-    const unsigned blocks = grid_for(n_cap, HIST_THREADS * HIST_KEYS, sm_count() * 4);
+template <int KEYS>
+static void launch_digit_hist_k(const olc_u32* keys, const olc_u32* n_dev, olc_u32 n_host, olc_u32 n_cap, olc_u32* hist,
+                                int passes, cudaStream_t s) {
+    const unsigned blocks = grid_for(n_cap, HIST_THREADS * KEYS, sm_count() * 4);
     if (passes == 1)
-        k_digit_hist<1><<<blocks, HIST_THREADS, 0, s>>>(keys, n_dev, n_host, hist);
+        k_digit_hist<1, KEYS><<<blocks, HIST_THREADS, 0, s>>>(keys, n_dev, n_host, hist);
     else if (passes == 2)
-        k_digit_hist<2><<<blocks, HIST_THREADS, 0, s>>>(keys, n_dev, n_host, hist);
+        k_digit_hist<2, KEYS><<<blocks, HIST_THREADS, 0, s>>>(keys, n_dev, n_host, hist);
     else if (passes == 3)
-        k_digit_hist<3><<<blocks, HIST_THREADS, 0, s>>>(keys, n_dev, n_host, hist);
+        k_digit_hist<3, KEYS><<<blocks, HIST_THREADS, 0, s>>>(keys, n_dev, n_host, hist);
     else
-        k_digit_hist<4><<<blocks, HIST_THREADS, 0, s>>>(keys, n_dev, n_host, hist);
+        k_digit_hist<4, KEYS><<<blocks, HIST_THREADS, 0, s>>>(keys, n_dev, n_host, hist);
+}
+
+void launch_digit_hist(const olc_u32* keys, const olc_u32* n_dev, olc_u32 n_host, olc_u32 n_cap, olc_u32* hist,
+                       int passes, cudaStream_t s) {
+    if (n_cap <= HIST_FEW)
+        launch_digit_hist_k<HIST_KEYS_FEW>(keys, n_dev, n_host, n_cap, hist, passes, s);
+    else
+        launch_digit_hist_k<HIST_KEYS>(keys, n_dev, n_host, n_cap, hist, passes, s);
 }
 
 void launch_scan_hist(const olc_u32* hist, olc_u32* base, int passes, olc_u32* tile_ctrs,

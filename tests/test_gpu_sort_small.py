@@ -97,3 +97,31 @@ def test_small_sort_among_other_work(cuda, olc, n):
     for out, _ in runs:
         np.testing.assert_array_equal(out[0].cpu().numpy().view(np.uint32), k[order])
         np.testing.assert_array_equal(out[1].cpu().numpy().view(np.uint32), order)
+
+
+@pytest.mark.parametrize("offset", [0, 3])
+@pytest.mark.parametrize("kind", ["equal", "runs", "random"])
+@pytest.mark.parametrize("n", [65537, 262143, 262144, 262145, 262161])
+def test_sorts_on_either_side_of_few_keys_per_thread(cuda, olc, n, kind, offset):
+    """The counts with 4 and with 16 keys per thread, at and off a 16-byte boundary,
+    where the last thread's share is not full."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    k = rng.integers(0, 1 << 30, n, dtype=np.uint64).astype(np.uint32)
+    if kind == "equal":
+        k[:] = k[0]
+    if kind == "runs":
+        k = np.sort(k)
+    order = np.argsort(k, kind="stable")
+    room = torch.zeros(n + 4, dtype=torch.int32, device=cuda)
+    kin = room[offset:offset + n]
+    kin.copy_(torch.from_numpy(k.view(np.int32).copy()))
+    kout, vout = (torch.zeros(n, dtype=torch.int32, device=cuda) for _ in range(2))
+    nbytes = olc.olc_sort_scratch_bytes(n, 30)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=cuda)
+    ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    _lib.check(olc.olc_stage_sort_pairs(ptr(kin), None, ptr(kout), ptr(vout), n, 30, ptr(scratch), nbytes, None))
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(kout.cpu().numpy().view(np.uint32), k[order])
+    np.testing.assert_array_equal(vout.cpu().numpy().view(np.uint32), order)
