@@ -495,10 +495,13 @@ __device__ __forceinline__ void atomic_min_nonneg_b(double* p, double v) {
 //
 // One atomic per row and value serialised on the few records (285,000 agents of
 // 16 members: 0.6 ms).  Rows of a simulation are contiguous after the sort, so
-// each warp takes a run of RAB_ROWS consecutive rows, sums the simulation at
+// each warp takes runs of consecutive rows, sums the simulation at
 // hand in registers (the histograms in its own shared-memory words) and adds to
-// the record only when the simulation changes and at the end of the run.
-constexpr olc_u32 RAB_ROWS = 512;
+// the record only when the simulation changes and at the end of the run.  A run is
+// the warp's share of the rows, RAB_LEAST to RAB_ROWS of them: always 512 left most of
+// the SMs without work (the whole collection of 200 members of 300 agents 36 us, so 13;
+// 16 of 18,000: 14.3 and 11.2; 4 of 60,000: 13.5 and 11.1).
+constexpr olc_u32 RAB_ROWS = 512, RAB_LEAST = 32;
 constexpr int RAB_WARPS = 8;
 
 __global__ void __launch_bounds__(32 * RAB_WARPS) k_reduce_agents_batch(
@@ -515,6 +518,7 @@ __global__ void __launch_bounds__(32 * RAB_WARPS) k_reduce_agents_batch(
     const olc_u32 warps = gridDim.x * RAB_WARPS, warp = blockIdx.x * RAB_WARPS + (threadIdx.x >> 5);
     olc_u32 cur = NONE, live = 0;  // the simulation at hand (the same in every lane)
     double sx = 0.0, sy = 0.0, sz = 0.0, sr2 = 0.0, mr = 0.0, cx = 0.0, cy = 0.0, cz = 0.0, bw = 1.0;
+    const olc_u32 share = min(max(((n + warps - 1) / warps + 31) / 32 * 32, RAB_LEAST), RAB_ROWS);  // rows of a run
     auto flush = [&]() {
         if (cur == NONE) return;
         OlcReductions* o = out + cur;
@@ -545,8 +549,8 @@ __global__ void __launch_bounds__(32 * RAB_WARPS) k_reduce_agents_batch(
         sx = sy = sz = sr2 = mr = 0.0;
         live = 0;
     };
-    for (olc_u64 first = (olc_u64)warp * RAB_ROWS; first < n; first += (olc_u64)warps * RAB_ROWS) {
-        const olc_u32 last = (olc_u32)(first + RAB_ROWS < n ? first + RAB_ROWS : n);
+    for (olc_u64 first = (olc_u64)warp * share; first < n; first += (olc_u64)warps * share) {
+        const olc_u32 last = (olc_u32)(first + share < n ? first + share : n);
         for (olc_u32 base = (olc_u32)first; base < last; base += 32) {
             const olc_u32 i = base + lane;
             const bool on = i < last && life[i < last ? i : base] == 0;
@@ -596,7 +600,7 @@ __global__ void __launch_bounds__(32 * RAB_WARPS) k_reduce_agents_batch(
 
 void launch_reduce_agents_batch(const BatchArgs& b, const ReduceArgs& a, const olc_u32* sim, const olc_u32* counters,
                                 olc_u32 n_cap, OlcReductions* out, cudaStream_t s) {
-    k_reduce_agents_batch<<<grid_cap(n_cap, RAB_ROWS * RAB_WARPS, sm_blocks(4)), 32 * RAB_WARPS, 0, s>>>(
+    k_reduce_agents_batch<<<grid_cap(n_cap, RAB_LEAST * RAB_WARPS, sm_blocks(4)), 32 * RAB_WARPS, 0, s>>>(
         a.x, a.y, a.z, a.state, sim, a.life, counters, b.sims, out);
 }
 

@@ -39,3 +39,10 @@ def test_member_reductions_match_their_rows(cuda, counts, storage):
                 v = snap["fields"][f].astype(np.float64)
                 np.testing.assert_allclose(red["field_mass"][f], v.sum(), rtol=4 * v.size * 2.0 ** -53)
                 assert red["field_min"][f] == v.min() and red["field_max"][f] == v.max()
+
+
+@pytest.mark.parametrize("counts", [(300,) * 40, (30,) * 80, (40_000, 20, 90_000, 33)])
+def test_reductions_with_shares_of_every_size(cuda, counts):
+    """Few rows, one 32-row run per warp; many, longer runs; members that change
+    within and between them."""
+    test_member_reductions_match_their_rows(cuda, counts, "f32")
