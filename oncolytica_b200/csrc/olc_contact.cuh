@@ -83,7 +83,7 @@ constexpr int CONTACT_RUNS = 18;
 //
 // A thread lists its runs, walks their rows two at a time (four loads in flight)
 // and lists the near rows; when a lane's list may overflow, and at the end, the
-// warp computes the listed pairs together.  Bound by the L1 data pipe (60 % busy:
+// warp computes the listed pairs together.  Bound by the L1 data pipe (70 % busy:
 // the records of ~10 bins per load) and the latency behind it; every byte of shared
 // memory per thread costs threads and L1.  1 M agents: 273 us, with 27 runs per
 // thread 306, with two-row loads of 32 bytes 323, computing the law in the walk 347.

@@ -434,7 +434,9 @@ bool make_field_maps16(FieldMaps16* m, void* a, void* b, const int dims[3], int 
     // deep tiles leave the SMs waiting).  us per BF16-SR substep with 8, 4, 2
     // and 1 planes: 256^3 27.8, 27.0, -, -; 200^3 20.8, 18.4, 19.4, -;
     // 160^3 16.2, 11.4, 10.8, 11.9; 256 x 256 x 64 -, 11.2, 9.3, 10.3;
-    // 128^3 -, -, 7.0, 6.3; 32^3 -, -, 3.3, 2.6.
+    // 128^3 -, -, 7.0, 6.3; 32^3 -, -, 3.3, 2.6.  The other encodings keep 8 planes: 4
+    // are faster at 160 x 150 x 170 (7.6 -> 5.8) and slower in batches (a step of 16
+    // members 2,012 -> 2,096 us); no rule between the two has been measured.
     m->tz = TZ;
     if (four_rows(encoding)) {
         int sms = 148, dev = 0;

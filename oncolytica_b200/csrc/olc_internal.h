@@ -141,7 +141,7 @@ struct MarchPlan {
     int lx = 0;              // lanes per row, 0: the march does not apply
     int w = 0;               // warps per CTA
     int gx = 0, gy = 0, gz = 0;  // grid
-    int zl = 0;              // planes per warp
+    int zl = 0;              // output planes per CTA
 };
 bool march_pays(const int dims[3]);
 bool make_march_plan(const int dims[3], float bval, int planes, MarchPlan* p, cuuint32_t box[3]);

@@ -5,9 +5,9 @@
 // tile of rows: input planes arrive by TMA in a ring of shared-memory slots,
 // and each step computes one plane of the intermediate field and one plane of
 // results from it.  A lane holds four consecutive x voxels of R rows of two
-// intermediate planes in registers; what bounds the pass is instruction issue
-// and the FP32 pipe (54 % and 46 % busy, 17.8 M warp instructions per pass on
-// 256^3 against 21.3 M for two one-substep passes), so:
+// intermediate planes in registers; what bounds the pass is the L1 data pipe,
+// instruction issue and the FP32 pipe (74, 57 and 47 % busy, 18.1 M warp instructions
+// per pass on 256^3 against 21.3 M for two one-substep passes), so:
 //   * R = 4 rows per lane: a row's y neighbours are the lane's own registers,
 //     but for the group's outer rows, which go through shared memory (one
 //     barrier per step, which also frees the oldest input slot).  Recomputing
@@ -22,7 +22,8 @@
 //   * Two copies of the step per loop and no more: a larger body missed the
 //     instruction cache (2.1 stalls per instruction with six copies).
 // Measured (us per substep, before -> after): 256^3 20.9 -> 15.6, 192^3 9.1 ->
-// 7.6, 128^3 5.2 -> 3.8, 100 x 100 x 256 6.1 -> 4.8.
+// 7.6, 128^3 5.2 -> 3.8 (a size that stays on chip unless pairs are asked for),
+// 100 x 100 x 256 6.1 -> 4.8.
 // Alternate passes march in opposite directions, so a pass starts on the planes
 // that the previous one wrote last, while they are in L2.
 #include "olc_internal.h"

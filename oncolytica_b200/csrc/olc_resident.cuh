@@ -6,8 +6,8 @@
 // and 9.7 at 117 x 75 x 131, whose rows no tensor map describes).  Here each
 // CTA of a cooperative grid (one per SM) keeps a tile of full rows in shared
 // memory, and the CTAs exchange only the tiles' outer rows after each substep
-// (whole field steps of 79, 88 and 21 substeps: 235 -> 93 us, 452 -> 165,
-// 203 -> 98).
+// (whole field steps of 79, 88 and 21 substeps: 232 -> 97 us, 451 -> 170,
+// 216 -> 100).
 //
 // Exchange without flags, fences or barriers: a substep's results are never
 // negative (the clamp), so the sign bit of a published word is free and carries
@@ -90,7 +90,7 @@ __device__ __forceinline__ void sts4(olc_u32 p, float4 v) {
 // memory (two copies of the tile and its ring of one row and one plane).  The same
 // words are reached by plain accesses and by the asm ones above, whose "memory"
 // clobbers keep the compiler from reordering the two.  What
-// bounds it is latency (the exchange, about 0.8 us) and, on larger tiles,
+// bounds it is latency (the exchange: a substep of 8^3 takes 0.65 us) and, on larger tiles,
 // instruction issue: the threads' addresses, faces and publications are worked
 // out once, before the substeps.
 template <int K, int NT, int RI, bool WRAP, class E>
